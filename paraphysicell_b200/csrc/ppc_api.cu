@@ -34,18 +34,48 @@ int fail(int rc, const std::string& msg)
 	return rc;
 }
 
-template <typename T>
-int alloc(ppc_state* s, T*& p, size_t count, bool zero = true)
+// Device arrays of a state: `want` collects them, `place` carves them out of
+// one block and clears those that start at zero with one memset (they lie
+// first; on the state's stream, since the legacy stream would not order with
+// it). One allocation instead of some eighty.
+struct arena
 {
-	size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
-	void* q = nullptr;
-	PPC_CUDA(cudaMalloc(&q, bytes));
-	if (zero) // on the state's stream (non-blocking: the legacy stream would not order with it)
-		PPC_CUDA(cudaMemsetAsync(q, 0, bytes, s->stream));
-	s->allocations.push_back({ q, bytes });
-	p = static_cast<T*>(q);
-	return PPC_OK;
-}
+	struct item
+	{
+		void** p;
+		size_t bytes;
+		bool zero;
+	};
+	std::vector<item> items;
+
+	template <typename T>
+	void want(T*& p, size_t count, bool zero = true)
+	{
+		items.push_back({ reinterpret_cast<void**>(&p), (std::max<size_t>(count, 1) * sizeof(T) + 255) & ~(size_t)255, zero });
+	}
+
+	int place(ppc_state* s)
+	{
+		size_t total = 0, cleared = 0;
+		for (const auto& it : items)
+		{
+			total += it.bytes;
+			cleared += it.zero ? it.bytes : 0;
+		}
+		char* q = nullptr;
+		PPC_CUDA(cudaMalloc(&q, total));
+		s->allocations.push_back({ q, total });
+		if (cleared)
+			PPC_CUDA(cudaMemsetAsync(q, 0, cleared, s->stream));
+		char* rest = q + cleared;
+		for (const auto& it : items)
+		{
+			*it.p = it.zero ? q : rest;
+			(it.zero ? q : rest) += it.bytes;
+		}
+		return PPC_OK;
+	}
+};
 
 #define PPC_TRY(x)                                                                                                     \
 	do                                                                                                                 \
@@ -153,6 +183,7 @@ int device_errors(ppc_state* s)
 // the bins no longer match the positions: the next step rebuilds them
 void invalidate_bins(ppc_state* s)
 {
+	s->skin_lists = false;
 	s->bins_valid = false;
 	s->bins_cond = false;
 }
@@ -320,6 +351,14 @@ bool only_kinematic(const ppc_agents* a)
 	return true;
 }
 
+double largest(const double* x, int32_t n)
+{
+	double m = 0;
+	for (int32_t i = 0; i < n; i++)
+		m = std::max(m, x[i]);
+	return m;
+}
+
 int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 {
 	const rep_info& R = s->reps[r];
@@ -332,6 +371,13 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 		for (int32_t i = 0; i < n; i++)
 			if (a->cell_definition_indices[i] < 0 || a->cell_definition_indices[i] >= D)
 				return fail(PPC_ERR_ARG, "cell definition index out of range");
+
+	// the bound on the interaction reach that admits steps over lists
+	if (a->radius || defaults)
+		s->reach_radius[r] = a->radius ? largest(a->radius, n) : kRadius;
+	if (a->relative_maximum_adhesion_distance || defaults)
+		s->reach_factor[r]
+			= a->relative_maximum_adhesion_distance ? largest(a->relative_maximum_adhesion_distance, n) : 1.25;
 
 	// an upload of kinematic fields only (positions, velocities, previous
 	// velocities, pressure, orientation) keeps the mesh when the positions it
@@ -466,6 +512,7 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 			s->bins_valid = false;
 			s->bins_cond = true;
 		}
+		s->skin_refresh = true;
 		// page-locked rows are copied by the queued DMA, so the call returns
 		// at once and the next step queues behind the copies; pageable rows
 		// are waited for, so the caller may reuse them on return
@@ -474,6 +521,7 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 		return PPC_OK;
 	}
 	invalidate_bins(s);
+	*s->pinned_skin = 1.f; // the fields that decide the skin may have changed
 	// slots were rewritten: the next rebuild counts by slot
 	PPC_CUDA(cudaMemsetAsync(v.order_valid, 0, sizeof(int32_t), s->stream));
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
@@ -745,6 +793,54 @@ int replay_steps(ppc_state* s, int k, bool phenotype, double p_divide, double p_
 	return PPC_OK;
 }
 
+constexpr int kListLeast = 4;	   // steps of a call that run over lists
+constexpr int kListSteps = 100000; // steps of one launch over lists
+
+// Whether a call's steps run over neighbour lists: the default launch shape
+// (an explicit other one asks for its own pass), and a mesh that leaves a
+// skin beyond the largest reach (by the uploaded fields; the device reports
+// the skin it found where radii changed there). The launch itself costs about
+// 13 us over its steps and making lists about as much as one scanning step,
+// so calls of a few steps keep the scanning passes: on 88,700 agents one step
+// after an upload takes 35 us over lists and 28 us scanning, four take about
+// the same, sixty 0.67 ms and 1.9 ms.
+bool use_lists(ppc_state* s, int32_t steps)
+{
+	if (!s->lists_fit || !s->queue || s->persistent || s->profiling || steps < kListLeast)
+		return false;
+	if (*static_cast<volatile float*>(s->pinned_skin) <= 0.f)
+		return false;
+	double voxel = 1e30;
+	for (const auto& R : s->reps)
+		for (int d = 0; d < s->dims; d++)
+			voxel = std::min(voxel, R.shape[d]);
+	for (int32_t r = 0; r < s->nreps; r++)
+		if (!(2.0 * s->reach_radius[r] * s->reach_factor[r] + 1.0 < voxel))
+			return false;
+	// a stream under capture is left to the replayed steps, which refuse it
+	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+	return cudaStreamIsCapturing(s->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+}
+
+int run_list_steps(ppc_state* s, int32_t steps)
+{
+	if (!s->skin_lists)
+	{
+		PPC_TRY(ensure_bins(s));
+		PPC_TRY(launch_lists(s));
+	}
+	for (int32_t done = 0; done < steps;)
+	{
+		const int32_t k = std::min(steps - done, (int32_t)kListSteps);
+		PPC_TRY(launch_list_steps(s, k));
+		done += k;
+	}
+	s->bins_valid = false; // the mesh stays that of the lists
+	s->bins_cond = false;
+	s->lists_stale = true;
+	return PPC_OK;
+}
+
 // after a call's last step: a download may run beside its rebuild while no
 // other kernel is launched
 int mark_ready(ppc_state* s)
@@ -764,6 +860,8 @@ int run_steps(ppc_state* s, int32_t steps, bool phenotype, double p_divide, doub
 		s->counts_known = false; // compaction and division change the counts
 	s->ready_pending = false;
 	s->ready_recorded = false;
+	if (!phenotype && !stochastic_springs(s) && use_lists(s, steps))
+		return run_list_steps(s, steps);
 	const bool graphs = s->use_graphs && !s->profiling;
 	// a rebuild the device decides on (after an upload of positions) rides
 	// at the head of the first replayed graph
@@ -810,6 +908,32 @@ int run_steps(ppc_state* s, int32_t steps, bool phenotype, double p_divide, doub
 	}
 	s->lists_stale = steps > 0 || s->lists_stale;
 	return mark_ready(s);
+}
+
+// The lists' arrays, about 1.4 KB per agent. A device without room for them
+// beside the state runs every step through the scanning passes.
+void alloc_lists(ppc_state* s)
+{
+	const size_t C = s->total_cap;
+	view& v = s->v;
+	v.nl_pool = 24 * (int64_t)C + 8192;
+	arena a;
+	a.want(v.nl_used, 1);
+	a.want(s->list_bar, 64);
+	a.want(v.lpos[0], C, false);
+	a.want(v.lpos[1], C, false);
+	a.want(v.lvprev, C, false);
+	a.want(v.lpress, C, false);
+	a.want(v.nlc, C, false);
+	a.want(v.nl_slab, C / 32 + 1, false);
+	a.want(v.nl, v.nl_pool, false);
+	a.want(v.nl_pair, v.nl_pool, false);
+	a.want(v.lspr, C * s->scap, false);
+	a.want(v.lcoef, C * s->scap, false);
+	a.want(v.tpos, C, false);
+	s->lists_fit = a.place(s) == PPC_OK;
+	if (!s->lists_fit)
+		cudaGetLastError(); // no room is not an error of the state
 }
 
 // grid of a mesh (validated: positive voxel shapes, maxs >= mins); sizes in
@@ -893,6 +1017,8 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 		}
 		R.inv_grid[0] = 1.0 / R.grid[0];
 		R.inv_grid[1] = 1.0 / R.grid[1];
+		for (int d = 0; d < 3; d++)
+			R.inv_shape[d] = 1.0 / std::max(R.shape[d], 1.0);
 		R.base = (int32_t)cap;
 		R.cap = capacities[r];
 		R.vox_base = vox;
@@ -940,13 +1066,11 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 	v.walls = params->virtual_wall_at_domain_edges;
 	v.auto_springs = params->automated_spring_adhesion != 0;
 	rep_info* reps = nullptr;
-	try_(alloc(s, reps, replicates));
-	v.reps = reps;
+	arena a;
+	a.want(reps, replicates);
 	// the error word sits right after the counters, so one copy brings both
-	try_(alloc(s, v.ctr, (size_t)replicates + 1));
-	if (rc == PPC_OK)
-		v.err = reinterpret_cast<int32_t*>(v.ctr + replicates);
-	try_(alloc(s, v.cursor, 1));
+	a.want(v.ctr, (size_t)replicates + 1);
+	a.want(v.cursor, 1);
 	v.nvox = (int32_t)vox;
 	{
 		// rebuild tiles of about 512 agents at full capacity, 64 to 4096 voxels
@@ -955,86 +1079,110 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 		v.tshift = std::min(12, std::max(6, sh));
 	}
 	v.ntiles = (int32_t)((vox + (1 << v.tshift) - 1) >> v.tshift);
-	try_(alloc(s, v.pos[0], C));
-	try_(alloc(s, v.pos[1], C));
-	try_(alloc(s, v.vel, C));
-	try_(alloc(s, v.vprev, C));
-	try_(alloc(s, v.prm, C));
-	try_(alloc(s, v.rmad, C));
-	try_(alloc(s, v.ec, C));
-	try_(alloc(s, v.arate, C));
-	try_(alloc(s, v.drate, C));
-	try_(alloc(s, v.pressure, C));
-	try_(alloc(s, v.vol, C));
-	try_(alloc(s, v.nvol, C));
-	try_(alloc(s, v.nrad, C));
-	try_(alloc(s, v.sarea, C));
-	try_(alloc(s, v.polarity, C));
-	try_(alloc(s, v.orient, C));
-	try_(alloc(s, v.aff, C * s->ndefs));
-	try_(alloc(s, v.def, C));
-	try_(alloc(s, v.maxatt, C));
-	try_(alloc(s, v.scnt, C));
-	try_(alloc(s, v.springs, C * s->scap));
-	try_(alloc(s, v.movable, C));
-	try_(alloc(s, v.flags, C));
-	try_(alloc(s, v.ids, C));
-	try_(alloc(s, v.rid, C));
-	try_(alloc(s, v.vstart, (size_t)vox + 1));
-	try_(alloc(s, v.key, C));
-	try_(alloc(s, v.tmp, C));
-	try_(alloc(s, v.vsc, C));
-	try_(alloc(s, v.tprev, (size_t)v.ntiles));
-	try_(alloc(s, v.tdelta, (size_t)v.ntiles));
-	try_(alloc(s, v.sdelta, ((size_t)v.ntiles + 1023) / 1024));
-	try_(alloc(s, v.chead, (size_t)v.ntiles * 32));
-	try_(alloc(s, v.cnext, C));
-	try_(alloc(s, v.porder, C));
-	try_(alloc(s, v.tfresh, C));
-	try_(alloc(s, v.params_changed, 1));
-	try_(alloc(s, v.copy_full, 1));
-	try_(alloc(s, v.recount, 1));
+	a.want(v.pos[0], C);
+	a.want(v.pos[1], C);
+	a.want(v.vel, C);
+	a.want(v.vprev, C);
+	a.want(v.prm, C);
+	a.want(v.rmad, C);
+	a.want(v.ec, C);
+	a.want(v.arate, C);
+	a.want(v.drate, C);
+	a.want(v.pressure, C);
+	a.want(v.vol, C);
+	a.want(v.nvol, C);
+	a.want(v.nrad, C);
+	a.want(v.sarea, C);
+	a.want(v.polarity, C);
+	a.want(v.orient, C);
+	a.want(v.aff, C * s->ndefs);
+	a.want(v.def, C);
+	a.want(v.maxatt, C);
+	a.want(v.scnt, C);
+	a.want(v.springs, C * s->scap);
+	a.want(v.movable, C);
+	a.want(v.flags, C);
+	a.want(v.ids, C);
+	a.want(v.rid, C);
+	a.want(v.vstart, (size_t)vox + 1);
+	a.want(v.key, C);
+	a.want(v.tmp, C);
+	a.want(v.vsc, C);
+	a.want(v.tprev, (size_t)v.ntiles);
+	a.want(v.tdelta, (size_t)v.ntiles);
+	a.want(v.sdelta, ((size_t)v.ntiles + 1023) / 1024);
+	a.want(v.chead, (size_t)v.ntiles * 32);
+	a.want(v.cnext, C);
+	a.want(v.porder, C);
+	a.want(v.tfresh, C);
+	a.want(v.params_changed, 1);
+	a.want(v.copy_full, 1);
+	a.want(v.recount, 1);
+	a.want(v.order_valid, 1);
+	a.want(v.binned, replicates);
+	a.want(v.moves_pending, 1);
+	a.want(v.appended, 1);
+	a.want(v.move_src, C); // -1: no pending move into the slot
+	a.want(v.sdel, C * s->scap);
+	a.want(v.first_end, C);
+	a.want(v.pos_changed, 1);
+	a.want(v.bin_active, 1);
+	a.want(v.barrier, 2);
+	a.want(v.sorted, C);
+	a.want(v.skey, C);
+	a.want(v.spos4, C);
+	a.want(v.spos4_next, C);
+	a.want(v.sprm4, C);
+	a.want(v.sposf, C);
+	a.want(v.sposf_next, C);
+	a.want(v.sprmf, C);
+	a.want(v.safff, C * s->ndefs);
+	a.want(v.saff, C * s->ndefs);
+	a.want(v.ncnt, C);
+	a.want(v.lctl, 8);
+	s->reach_radius.assign(replicates, kRadius);
+	s->reach_factor.assign(replicates, 1.25);
+	a.want(v.bad, C);
+	a.want(v.divl, C);
+	a.want(v.moves, 2 * C);
+	a.want(v.nmoves, replicates);
+	a.want(v.draw_epoch, replicates);
+	try_(rc == PPC_OK ? a.place(s) : rc);
+	if (rc == PPC_OK)
+	{
+		v.reps = reps;
+		v.err = reinterpret_cast<int32_t*>(v.ctr + replicates);
+		// its own block: ppc_set_neighbor_capacity replaces it
+		void* lists = nullptr;
+		const size_t bytes = C * s->ncap * sizeof(int32_t);
+		if (cudaMalloc(&lists, bytes) != cudaSuccess)
+			rc = fail(PPC_ERR_CUDA, "cudaMalloc failed");
+		else
+		{
+			s->allocations.push_back({ lists, bytes });
+			v.nidx = static_cast<int32_t*>(lists);
+		}
+	}
 	if (rc == PPC_OK && cudaMemsetAsync(v.chead, 0xff, sizeof(int32_t) * (size_t)v.ntiles * 32, s->stream) != cudaSuccess)
 		rc = fail(PPC_ERR_CUDA, "cudaMemset failed");
-	try_(alloc(s, v.order_valid, 1));
-	try_(alloc(s, v.binned, replicates));
-	try_(alloc(s, v.moves_pending, 1));
-	try_(alloc(s, v.appended, 1));
-	try_(alloc(s, v.move_src, C)); // -1: no pending move into the slot
-	try_(alloc(s, v.sdel, C * s->scap));
-	try_(alloc(s, v.first_end, C));
-	try_(alloc(s, v.pos_changed, 1));
-	try_(alloc(s, v.bin_active, 1));
-	try_(alloc(s, v.barrier, 2));
 	if (rc == PPC_OK && cudaMemsetAsync(v.first_end, 0x7f, sizeof(int32_t) * std::max<size_t>(C, 1), s->stream) != cudaSuccess)
 		rc = fail(PPC_ERR_CUDA, "cudaMemset failed");
 	if (rc == PPC_OK && cudaMemsetAsync(v.move_src, 0xff, sizeof(int32_t) * std::max<size_t>(C, 1), s->stream) != cudaSuccess)
 		rc = fail(PPC_ERR_CUDA, "cudaMemset failed");
-	try_(alloc(s, v.sorted, C));
-	try_(alloc(s, v.skey, C));
-	try_(alloc(s, v.spos4, C));
-	try_(alloc(s, v.spos4_next, C));
-	try_(alloc(s, v.sprm4, C));
-	try_(alloc(s, v.sposf, C));
-	try_(alloc(s, v.sposf_next, C));
-	try_(alloc(s, v.sprmf, C));
-	try_(alloc(s, v.safff, C * s->ndefs));
-	try_(alloc(s, v.saff, C * s->ndefs));
-	try_(alloc(s, v.ncnt, C));
-	try_(alloc(s, v.nidx, C * s->ncap, false));
-	try_(alloc(s, v.bad, C));
-	try_(alloc(s, v.divl, C));
-	try_(alloc(s, v.moves, 2 * C));
-	try_(alloc(s, v.nmoves, replicates));
-	try_(alloc(s, v.draw_epoch, replicates));
+	if (rc == PPC_OK)
+		alloc_lists(s);
 	s->host_count.assign(replicates, 0);
 	if (rc == PPC_OK
-		&& cudaHostAlloc(reinterpret_cast<void**>(&s->pinned_ctr), sizeof(rep_counters) * (replicates + 1),
-						 cudaHostAllocDefault)
+		&& cudaHostAlloc(reinterpret_cast<void**>(&s->pinned_ctr), sizeof(rep_counters) * (replicates + 2),
+						 cudaHostAllocMapped)
 			   != cudaSuccess)
 		rc = fail(PPC_ERR_CUDA, "cudaHostAlloc failed");
 	if (rc == PPC_OK)
+	{
 		s->pinned_err = reinterpret_cast<int32_t*>(s->pinned_ctr + replicates);
+		s->pinned_skin = reinterpret_cast<float*>(s->pinned_ctr + replicates + 1);
+		*s->pinned_skin = 1.f;
+	}
 	if (rc == PPC_OK)
 	{
 		std::vector<int32_t> rid(C, 0);
@@ -1223,6 +1371,9 @@ int ppc_upload(ppc_state* s, int32_t r, const ppc_agents* a)
 	PPC_CUDA(cudaMemcpyAsync(&s->v.ctr[r], &c, sizeof c, cudaMemcpyHostToDevice, s->stream));
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
 	s->lists_stale = false;
+	s->skin_reset = true;
+	if (s->lost && s->lists_fit)
+		PPC_CUDA(cudaMemsetAsync(s->list_bar, 0, 64 * sizeof(unsigned long long), s->stream));
 	s->lost = false;
 	return transfer_in(s, r, a, true);
 }

@@ -60,6 +60,7 @@ struct rep_info
 	int32_t maxs_int[3], mins_int[3];
 	float fmargin;	  // bound on the FP32 distance error of positions relative to mins (um)
 	double inv_grid[2]; // 1 / grid[0], 1 / grid[1]: voxel coordinates of a key without integer division
+	double inv_shape[3]; // 1 / shape
 };
 
 // per-replicate device counters
@@ -185,6 +186,22 @@ struct view
 	int32_t* ncnt;
 	int32_t* nidx;
 
+	// neighbour lists that outlive a step (ppc_lists.cuh), in the key order of
+	// the mesh they were made from: list entries are positions in that order
+	double4* lpos[2];	 // current position and order word (voxel key, complement of the slot), double-buffered
+	double4* lvprev;	 // previous velocity
+	double* lpress;		 // pressure of the last step
+	int32_t* nlc;		 // [C] list length
+	int64_t* nl_slab;	 // [C / 32] start of the entries of 32 agents (entry k of agent l at k * 32 + l), or -1
+	int2* nl;			 // [nl_pool] neighbour with whether it is movable, and the pair's reach (float)
+	double4* nl_pair;	 // [nl_pool] what the pair code needs of the two agents' fields
+	int64_t nl_pool;
+	unsigned long long* nl_used;
+	int32_t* lspr;		 // [scap * C] spring partners' positions in the key order
+	double* lcoef;		 // [scap * C] the springs' coefficients
+	int32_t* tpos;		 // [C] position of each slot in the key order
+	int32_t* lctl;		 // control words (LCTL_*)
+
 	int32_t* bad;	  // per replicate: removal candidates (local indices), C entries total at base_r
 	int32_t* divl;	  // per replicate: division list, same layout
 	int32_t* moves;	  // per replicate: (dst, src) pairs of the compaction, 2*C at 2*base_r
@@ -195,6 +212,18 @@ struct view
 
 	ix_columns ix;
 	mot_columns mot;
+};
+
+// words of view::lctl
+enum : int
+{
+	LCTL_DIRTY = 0, // the lists are past their skin: rebuild before the next step
+	LCTL_REACH = 1, // bits of the largest interaction reach (float, rounded up) at the last rebuild
+	LCTL_CAP = 2,	// bits of the largest skin the lists being made may take
+	LCTL_WANT = 3,	// the same for the next lists: lowered where a pool of entries was too small
+	LCTL_BUILT = 4, // bits of the skin of the lists in use
+	LCTL_FIT = 5,	// every warp has its lists
+	LCTL_LEFT = 6	// steps a launch over lists left to the one behind it
 };
 
 struct buffer
@@ -281,6 +310,18 @@ struct ppc_state
 	bool counts_known = false;	  // host_count holds the device counts (no count-changing work since)
 	bool zero_copy = false;		  // pinned host rows are read and written by kernels over the bus
 	bool lists_stale = false;	  // a fused step ran since the neighbour lists were built
+	// the lists that outlive a step: whether they and their key-ordered copies
+	// hold, apart from an upload of positions or velocities (skin_refresh)
+	bool skin_lists = false;
+	bool skin_refresh = false;
+	bool skin_reset = true;		  // a full upload since lists were made
+	bool lists_fit = false;		  // the device had room for the lists
+	int lcur = 0;				  // lpos buffer that holds the positions
+	int bar_set = 0;			  // barrier words of the next list launch
+	unsigned long long* list_bar = nullptr; // [2 sets * 2 words * 16]
+	bool list_attr[2][2] = {};	  // the list kernels' shared-memory limits are set (per precision and kernel)
+	std::vector<double> reach_radius, reach_factor; // per replicate: largest uploaded radius and rmad
+	float* pinned_skin = nullptr; // skin of the lists in use, written by the device (0: none)
 	int64_t launches = 0;
 	int max_grid_blocks = 0;
 	int sm_count = 148;
@@ -366,6 +407,9 @@ int launch_spring_updates(ppc_state* s);
 int launch_positions(ppc_state* s);
 int launch_fused(ppc_state* s);
 int launch_step_persistent(ppc_state* s);
+// neighbour lists from the current mesh, and `steps` steps over them
+int launch_lists(ppc_state* s);
+int launch_list_steps(ppc_state* s, int steps);
 int launch_compact(ppc_state* s, bool phenotype_pass, bool fold = false, bool produced = false);
 int launch_mark_remove(ppc_state* s);
 int launch_divide(ppc_state* s);

@@ -6,6 +6,8 @@
 // written in the reference's order. Each kernel cites the reference lines it
 // replaces.
 #include <cuda_runtime.h>
+
+#include <algorithm>
 #include <utility>
 
 #include "../../include/ppc_draws.h"
@@ -327,7 +329,10 @@ __global__ void __launch_bounds__(kThreads) k_bin_count(view v, int cur, int con
 	const int t = blockIdx.x * blockDim.x + threadIdx.x;
 	const bool active = !conditional || *v.pos_changed != 0 || *v.moves_pending != 0 || *v.appended != 0;
 	if (t == 0)
+	{
 		*v.bin_active = active ? 1 : 0;
+		v.lctl[LCTL_REACH] = 0;
+	}
 	if (!active || (produced && *v.recount == 0))
 		return;
 	bin_count_body(v, cur, t);
@@ -414,10 +419,11 @@ __device__ __forceinline__ int2 place_item(const view& v, const place_smem& sm, 
 // exclusive scan of cnt[0, 4 ceil(nv / 4)) in place: each warp scans a
 // contiguous chunk of 16-byte groups in rows of 32 groups (no bank
 // conflicts), then the warps' totals are added
+// (THREADS 0: the block size is known at run time only)
 template <int THREADS>
 __device__ __forceinline__ void place_scan(place_smem& sm, int nv)
 {
-	constexpr int NW = THREADS / 32;
+	const int NW = (THREADS ? THREADS : (int)blockDim.x) / 32;
 	const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 	int4* c4 = reinterpret_cast<int4*>(sm.cnt);
 	const int nq = (nv + 3) >> 2;
@@ -478,9 +484,10 @@ __device__ __forceinline__ void place_scan(place_smem& sm, int nv)
 // fields follow in k_bin_copy, which also readies the counters for the next
 // rebuild (bin_finish).
 // `on`: the rebuild runs (bin_active; the same for the whole block).
-template <int THREADS>
+template <int BLOCK>
 __device__ __forceinline__ void bin_order_tile(const view& v, int b, place_smem& sm, int on)
 {
+	const int THREADS = BLOCK ? BLOCK : (int)blockDim.x;
 	const int tid = threadIdx.x, lane = tid & 31;
 	const int sh = v.tshift;
 	const int k0 = b << sh;
@@ -585,7 +592,7 @@ __device__ __forceinline__ void bin_order_tile(const view& v, int b, place_smem&
 		// was and stays empty at the same start keeps them
 		if (n > 0)
 		{
-			place_scan<THREADS>(sm, nv);
+			place_scan<BLOCK>(sm, nv);
 			int4* vs4 = reinterpret_cast<int4*>(v.vstart + k0); // k0 is a multiple of 64
 			const int4* c4 = reinterpret_cast<const int4*>(sm.cnt);
 			for (int q = tid; q < nv >> 2; q += THREADS)
@@ -3820,6 +3827,8 @@ __global__ void __launch_bounds__(kPersistThreads) k_step_persistent(view v, int
 	bin_finish(v, blockIdx.x * kPersistThreads + threadIdx.x, nb * kPersistThreads);
 }
 
+#include "ppc_lists.cuh"
+
 } // namespace
 
 // ---------------------------------------------------------------------------
@@ -3863,6 +3872,7 @@ void flip_sorted_positions(ppc_state* s)
 // download can run beside the rest of the rebuild
 int launch_bin(ppc_state* s, bool conditional, bool ready, bool produced)
 {
+	s->skin_lists = false; // the key order the lists refer to changes
 	const int b = blocks_for(s->total_cap, kThreads);
 	pdl(k_bin_count, b, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur, conditional ? 1 : 0, produced ? 1 : 0);
 	if (ready)
@@ -3949,6 +3959,7 @@ int launch_springs(ppc_state* s)
 // next rebuild's k_bin_copy rewrites every key-ordered field
 int mark_fields_changed(ppc_state* s)
 {
+	s->skin_lists = false;
 	PPC_CUDA(cudaMemsetAsync(s->v.params_changed, 1, sizeof(int32_t), s->stream));
 	return PPC_OK;
 }
@@ -4016,6 +4027,16 @@ static int fused_opts(ppc_state* s)
 	return (s->params.virtual_wall_at_domain_edges ? FUSED_WALLS : 0)
 		   | ((s->has_springs && s->params.automated_spring_adhesion) ? FUSED_SPRINGS : 0)
 		   | (s->vel_dirty ? FUSED_VEL : 0) | (s->produce ? FUSED_PRODUCE : 0);
+}
+
+// the smallest voxel edge of the state's meshes
+static float list_voxel(ppc_state* s)
+{
+	double e = 1e30;
+	for (const auto& R : s->reps)
+		for (int d = 0; d < s->dims; d++)
+			e = std::min(e, R.shape[d]);
+	return (float)e;
 }
 
 // the staged pass's staging capacity (float4 positions) and dynamic shared bytes
@@ -4169,6 +4190,104 @@ int launch_step_persistent(ppc_state* s)
 	if (rc != PPC_OK)
 		return rc;
 	s->cur ^= 1;
+	s->vel_dirty = false;
+	return PPC_OK;
+}
+
+int launch_lists(ppc_state* s)
+{
+	const int springs = (s->has_springs && s->params.automated_spring_adhesion) ? 1 : 0;
+	const float voxel = list_voxel(s);
+	pdl(k_list_prepare, blocks_for(s->total_cap, kThreads), kThreads, 0, PPC_LAUNCH(s), s->v,
+		s->skin_reset ? 1 : 0);
+	auto k = s->dims == 1 ? k_list_build<1> : (s->dims == 2 ? k_list_build<2> : k_list_build<3>);
+	pdl(k, blocks_for(s->total_cap, 128), 128, 0, PPC_LAUNCH(s), s->v, s->cur, s->lcur, springs, voxel,
+		s->pinned_skin);
+	PPC_CHECK_LAUNCH();
+	s->skin_lists = true;
+	s->skin_refresh = false;
+	s->skin_reset = false;
+	return PPC_OK;
+}
+
+// Threads per block: one thread per agent while the grid of one block per SM
+// holds them, so that no thread takes two agents in turn; a warp multiple.
+static int list_threads(ppc_state* s)
+{
+	const int per_sm = (s->total_cap + s->sm_count - 1) / s->sm_count;
+	return std::min(kListThreads, std::max(128, (per_sm + 31) / 32 * 32));
+}
+
+template <int DIMS, bool F32, bool RESIDENT, bool LISTED, int MOST>
+static int list_launch_form(ppc_state* s, list_args a, int T)
+{
+	a.bar = s->list_bar + 32 * s->bar_set;
+	a.bar_next = s->list_bar + 32 * (s->bar_set ^ 1);
+	s->bar_set ^= 1;
+	auto k = k_list_steps<DIMS, F32, RESIDENT, LISTED, MOST>;
+	const size_t warps = T / 32, step = warps * sizeof(list_step_warp);
+	const size_t entry = (size_t)T * (sizeof(double4) + sizeof(int2));
+	a.cached = RESIDENT ? (int)std::min<size_t>(16, (kListSmem - step) / entry) : 0;
+	const size_t dyn = std::max({ sizeof(place_smem), warps * sizeof(list_warp), step + a.cached * entry,
+								  (size_t)kSortCap * sizeof(int32_t) });
+	if (!s->list_attr[F32][LISTED])
+	{
+		int per_sm = 0;
+		PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+		PPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, T, dyn));
+		if (per_sm < 1)
+			return cuda_fail(cudaErrorInvalidConfiguration, "steps over lists: no block fits an SM");
+		s->list_attr[F32][LISTED] = true;
+	}
+	cudaLaunchConfig_t cfg {};
+	cfg.gridDim = dim3(std::min(s->sm_count, blocks_for(s->total_cap, T)));
+	cfg.blockDim = dim3(T);
+	cfg.dynamicSmemBytes = dyn;
+	cfg.stream = PPC_LAUNCH(s);
+	cudaLaunchAttribute at[1];
+	at[0].id = cudaLaunchAttributeCooperative;
+	at[0].val.cooperative = 1;
+	cfg.attrs = at;
+	cfg.numAttrs = 1;
+	PPC_CUDA(cudaLaunchKernelEx(&cfg, k, s->v, a));
+	return PPC_OK;
+}
+
+template <int DIMS, bool F32>
+static int list_launch(ppc_state* s, const list_args& a)
+{
+	const int T = list_threads(s);
+	const int rc = (int64_t)T * s->sm_count < s->total_cap
+					   ? list_launch_form<DIMS, F32, false, true, kListLoop>(s, a, kListLoop)
+					   : (T <= kListFew ? list_launch_form<DIMS, F32, true, true, kListFew>(s, a, T)
+										: list_launch_form<DIMS, F32, true, true, kListThreads>(s, a, T));
+	return rc != PPC_OK ? rc : list_launch_form<DIMS, F32, false, false, kListLoop>(s, a, kListLoop);
+}
+
+int launch_list_steps(ppc_state* s, int steps)
+{
+	list_args a {};
+	a.limit = 1LL << 25; // about 20 s of polls
+	a.opts = fused_opts(s);
+	a.steps = steps;
+	a.p = s->lcur;
+	a.cur = s->cur;
+	a.refresh = s->skin_refresh ? 1 : 0;
+	a.springs = s->has_springs ? 1 : 0;
+	a.voxel = list_voxel(s);
+	a.skin_out = s->pinned_skin;
+	const bool f32 = s->precision == PPC_FP32_FORCE;
+	int rc;
+	if (s->dims == 1)
+		rc = f32 ? list_launch<1, true>(s, a) : list_launch<1, false>(s, a);
+	else if (s->dims == 2)
+		rc = f32 ? list_launch<2, true>(s, a) : list_launch<2, false>(s, a);
+	else
+		rc = f32 ? list_launch<3, true>(s, a) : list_launch<3, false>(s, a);
+	if (rc != PPC_OK)
+		return rc;
+	s->lcur ^= steps & 1;
+	s->skin_refresh = false;
 	s->vel_dirty = false;
 	return PPC_OK;
 }
