@@ -563,7 +563,7 @@ int ppc_get_profile(ppc_state* s, double* fused_ms, int64_t* fused_launches);
 
 /* ---- binning without allocation ------------------------------------------ */
 
-/* Limits of the fixed scratch of ppc_bin_agents_noalloc (about 5.8 MB of
+/* Limits of the fixed scratch of ppc_bin_agents_noalloc (about 10.5 MB of
  * device memory reserved on every GPU that loads the library). */
 #define PPC_NOALLOC_MAX_AGENTS 131072
 #define PPC_NOALLOC_MAX_VOXELS 1048576

@@ -1,0 +1,44 @@
+"""ppc_bin_agents_noalloc at the sizes where its kernels change path: voxels
+with up to 24 agents (their chain), more (a block's sort) and more than 4096
+(rank counting), partial tiles, and buffers that are only 4-byte aligned."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from paraphysicell_b200 import build
+from paraphysicell_b200.abi import Mesh
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shift", [0, 1, 3])
+@pytest.mark.parametrize("clump,spread,side", [(1, 0, 1), (24, 300, 7), (25, 300, 7), (4096, 1000, 17),
+                                               (4097, 77, 16), (60, 131072 - 60, 101)])
+def test_crowded_voxels(clump, spread, side, shift):
+    import torch
+
+    from paraphysicell_b200 import device
+
+    build.ensure_built()
+    L = device.lib()
+    L.ppc_bin_agents_noalloc.argtypes = [C.POINTER(Mesh), C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
+    rng = np.random.default_rng(clump)
+    n = clump + spread
+    pos = rng.random((n, 3)) * 30 * side
+    pos[rng.permutation(n)[:clump]] = 30 * (side // 2) + rng.random((clump, 3)) * 29
+    mesh = Mesh.make(3, (0, 0, 0), (30 * side,) * 3)
+    key = (pos / 30.0).astype(np.int64)
+    key = key[:, 0] + side * (key[:, 1] + side * key[:, 2])
+    want_counts = np.bincount(key, minlength=side ** 3)
+    want_agents = np.lexsort((-np.arange(n), key))
+    dev = torch.from_numpy(pos.ravel()).cuda()
+    counts = torch.full((side ** 3 + shift,), -7, dtype=torch.int32, device="cuda")
+    agents = torch.full((n + shift,), -7, dtype=torch.int32, device="cuda")
+    for _ in range(2):
+        rc = L.ppc_bin_agents_noalloc(C.byref(mesh), dev.data_ptr(), n, counts[shift:].data_ptr(),
+                                      agents[shift:].data_ptr(), torch.cuda.current_stream().cuda_stream)
+        assert rc == 0, L.ppc_last_error()
+        assert np.array_equal(counts.cpu().numpy()[shift:], want_counts)
+        assert np.array_equal(agents.cpu().numpy()[shift:], want_agents)
+        assert (counts[:shift] == -7).all() and (agents[:shift] == -7).all()
