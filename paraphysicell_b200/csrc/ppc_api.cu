@@ -671,7 +671,8 @@ int enqueue_step(ppc_state* s, bool phenotype, double p_divide, double p_death, 
 {
 	if (s->persistent && !phenotype)
 		return launch_step_persistent(s);
-	// the compaction right before the rebuild leaves its moves to k_bin_count;
+	// a compaction leaves its moves to the kernel that visits every agent
+	// after it: k_phenotype, or k_bin_count of the rebuild;
 	// in a step without the phenotype update the fused passes -3 and -4 also
 	// make the count's entries, which hold unless the compaction removes agents
 	const bool produce = !phenotype && (s->flat || s->queue);
@@ -679,12 +680,10 @@ int enqueue_step(ppc_state* s, bool phenotype, double p_divide, double p_death, 
 	const int rc_fused = launch_fused(s);
 	s->produce = false;
 	PPC_TRY(rc_fused);
-	PPC_TRY(launch_compact(s, false, !phenotype, produce));
+	PPC_TRY(launch_compact(s, false, true, produce));
 	if (phenotype)
 	{
-		PPC_TRY(launch_flag_by_draws(s, p_divide, p_death));
-		PPC_TRY(launch_divide(s));
-		PPC_TRY(launch_mark_remove(s));
+		PPC_TRY(launch_phenotype(s, true, p_divide, p_death));
 		PPC_TRY(launch_compact(s, true, true));
 	}
 	PPC_TRY(launch_bin(s, false, last, produce));
@@ -705,12 +704,10 @@ int enqueue_step_separate(ppc_state* s, bool phenotype, double p_divide, double 
 	PPC_TRY(launch_springs(s));
 	PPC_TRY(launch_positions(s));
 	PPC_TRY(launch_mark_remove(s));
-	PPC_TRY(launch_compact(s, false, !phenotype));
+	PPC_TRY(launch_compact(s, false, true));
 	if (phenotype)
 	{
-		PPC_TRY(launch_flag_by_draws(s, p_divide, p_death));
-		PPC_TRY(launch_divide(s));
-		PPC_TRY(launch_mark_remove(s));
+		PPC_TRY(launch_phenotype(s, true, p_divide, p_death));
 		PPC_TRY(launch_compact(s, true, true));
 	}
 	PPC_TRY(launch_bin(s, false, last));
@@ -1535,8 +1532,7 @@ int ppc_update_cell_container_for_phenotype(ppc_state* s)
 		return fail(PPC_ERR_ARG, "null state");
 	s->counts_known = false;
 	PPC_TRY(ensure_lists(s));
-	PPC_TRY(launch_divide(s));
-	PPC_TRY(launch_mark_remove(s));
+	PPC_TRY(launch_phenotype(s, false, 0, 0));
 	PPC_TRY(launch_compact(s, true));
 	invalidate_bins(s);
 	return finish(s);

@@ -158,8 +158,9 @@ struct view
 	int32_t* recount;	// the compaction removed agents: the rebuild's count recomputes every entry
 	int32_t* order_valid; // 1 once a rebuild has set `sorted` (cleared by uploads)
 	int32_t* binned;	  // [replicates] live count at the last rebuild (the slots `sorted` lists)
-	int32_t* move_src;	  // [C] tail slot whose agent the next k_bin_count moves into this hole, or -1
-	int32_t* moves_pending; // a folded compaction left moves for the next k_bin_count
+	int32_t* move_src;	  // [C] tail slot whose agent k_phenotype or the next k_bin_count moves into this hole, -1, or
+						  // -2 (kMoved): the slot's fields changed since the last rebuild
+	int32_t* moves_pending; // a folded compaction left moves for them
 	int32_t* appended;		// agents were appended (division) since the last rebuild
 	uint8_t* sdel;		  // [C*S] spring marked for detachment this step
 	int32_t* first_end;	  // [C] INT32_MAX between spring attachment passes
@@ -412,7 +413,7 @@ int launch_lists(ppc_state* s);
 int launch_list_steps(ppc_state* s, int steps);
 int launch_compact(ppc_state* s, bool phenotype_pass, bool fold = false, bool produced = false);
 int launch_mark_remove(ppc_state* s);
-int launch_divide(ppc_state* s);
+int launch_phenotype(ppc_state* s, bool draws, double p_divide, double p_death);
 int launch_flag_by_draws(ppc_state* s, double p_divide, double p_death);
 int launch_count_flags(ppc_state* s, int32_t r, int32_t flag, int32_t* count);
 

@@ -218,6 +218,7 @@ constexpr int kSuperShift = 10;	 // tiles per entry of sdelta: 1024
 constexpr int kPlaceThreads = 256;
 constexpr int kPlaceList = 1024; // agents of a tile listed in shared memory; the rest in global scratch
 constexpr int kMaxTileShift = 12;
+constexpr int32_t kFresh = 1 << 30; // porder: the slot's fields changed (slots are fewer: an agent takes over 500 bytes)
 constexpr int kOrderBatch = 4;  // previous-order entries a thread of k_bin_order loads at once
 
 // the voxel key of slot s of replicate r at positions pos[cur]
@@ -231,16 +232,24 @@ __device__ __forceinline__ int32_t voxel_key(const view& v, int cur, int s, int 
 	return (int32_t)(R.vox_base + c0 + (int64_t)R.grid[0] * (c1 + (int64_t)R.grid[1] * c2));
 }
 
-// a hole the compaction plan filled takes its tail agent first
-__device__ __forceinline__ void apply_move(const view& v, int cur, int s)
+// A hole the compaction plan filled takes its tail agent first. True where
+// the slot's agent or its fields are not those of the last rebuild (a move
+// now or earlier, or kMoved left by the division): its key-ordered copies are
+// rewritten. A tail agent's own mark goes with it, and so never outlives it.
+constexpr int32_t kMoved = -2;
+
+__device__ __forceinline__ bool apply_move(const view& v, int cur, int s)
 {
 	const int src = v.move_src[s];
+	if (src == -1)
+		return false;
 	if (src >= 0)
 	{
 		move_agent(v, cur, s, src);
-		v.move_src[s] = -1;
-		*v.params_changed = 1; // the slot's agent changed: its key-ordered copies are rewritten
+		v.move_src[src] = -1;
 	}
+	v.move_src[s] = -1;
+	return true;
 }
 
 // pushes slot q onto a mover chain of the tile of `key`
@@ -285,12 +294,11 @@ __device__ __forceinline__ void bin_count_body(const view& v, int cur, int t)
 		int r, local;
 		if ((unsigned)q < (unsigned)v.total_cap && live(v, q, r, local))
 		{
-			if (moves)
-				apply_move(v, cur, q);
+			const bool fresh = moves && apply_move(v, cur, q);
 			const int32_t key = voxel_key(v, cur, q, r);
 			v.key[q] = key;
 			if ((key >> sh) == (okey >> sh))
-				e = make_int2(q, key);
+				e = make_int2(q | (fresh ? kFresh : 0), key);
 			else
 			{
 				chain_push(v, q, key);
@@ -557,8 +565,8 @@ __device__ __forceinline__ void bin_order_tile(const view& v, int b, place_smem&
 					at = atomicAdd(&sm.n, __popc(m));
 				at = __shfl_sync(0xffffffffu, at, 0);
 				if (keep)
-					place_store(v, sm, base, at + __popc(m & ((1u << lane) - 1)), e[k].x,
-								lv | (i + 1 < kPrevLimit ? (i + 1) << kVoxelBits : 0));
+					place_store(v, sm, base, at + __popc(m & ((1u << lane) - 1)), e[k].x & ~kFresh,
+								lv | (i + 1 < kPrevLimit && !(e[k].x & kFresh) ? (i + 1) << kVoxelBits : 0));
 			}
 		}
 	if (tid < kChains && chain >= 0)
@@ -2863,6 +2871,15 @@ __device__ void compact_plan_rep(const view& v, int r, int phenotype_pass, int s
 								 int32_t* sh)
 {
 	rep_counters& C = v.ctr[r];
+	if (phenotype_pass && threadIdx.x == 0)
+	{
+		// the daughters appended by k_divide_apply join the replicate
+		C.count += C.ndiv;
+		C.divisions += C.ndiv;
+		C.next_id += C.ndiv;
+		C.ndiv = 0;
+		v.draw_epoch[r]++;
+	}
 	const int nb = min(C.nbad, v.reps[r].cap);
 	if (nb == 0)
 	{
@@ -2890,8 +2907,25 @@ __device__ void compact_plan_rep(const view& v, int r, int phenotype_pass, int s
 	const int base = v.reps[r].base;
 	int32_t* B = v.bad + base;
 	block_sort(B, nb, sh);
+	// the candidates and whether each is flagged (a death), in shared memory:
+	// the serial loop below is a chain of such reads. 1 M agents, about 50
+	// removals, cold caches: 38 us with both in global memory, 20 us so.
+	const bool in_shared = nb <= kSortCap;
+	if (in_shared)
+	{
+		for (int k = threadIdx.x; k < nb; k += blockDim.x)
+		{
+			const int h = B[k];
+			sh[k] = h << 1 | (v.flags[base + h] == PPC_FLAG_TO_REMOVE ? 1 : 0);
+		}
+		__syncthreads();
+	}
 	if (threadIdx.x != 0)
 		return;
+	auto hole = [&](int k) { return in_shared ? sh[k] >> 1 : B[k]; };
+	auto dead = [&](int k) {
+		return in_shared ? (sh[k] & 1) != 0 : v.flags[base + B[k]] == PPC_FLAG_TO_REMOVE;
+	};
 
 	const int nvisit = phenotype_pass ? C.nvisit : C.count;
 	const int cnt0 = C.count;
@@ -2902,13 +2936,14 @@ __device__ void compact_plan_rep(const view& v, int r, int phenotype_pass, int s
 	int32_t* moves = v.moves + 2 * (int64_t)base;
 	for (int bi = 0; bi < nb; bi++)
 	{
-		const int h = B[bi];
+		const int h = hole(bi);
 		if (h >= nvisit || h >= cnt)
 			break;
-		int occ = h; // original index of the agent now in slot h
+		int occ = h;   // original index of the agent now in slot h
+		int cand = bi; // and its place among the candidates
 		while (true)
 		{
-			deaths += v.flags[base + occ] == PPC_FLAG_TO_REMOVE;
+			deaths += dead(cand);
 			const int last = cnt - 1;
 			if (springs)
 			{
@@ -2931,10 +2966,11 @@ __device__ void compact_plan_rep(const view& v, int r, int phenotype_pass, int s
 				break;
 			}
 			occ = last;
-			while (ti >= 0 && B[ti] > last)
+			while (ti >= 0 && hole(ti) > last)
 				ti--;
-			if (!(ti >= 0 && B[ti] == last))
+			if (!(ti >= 0 && hole(ti) == last))
 				break;
+			cand = ti;
 		}
 		if (occ >= 0)
 		{
@@ -3417,7 +3453,14 @@ __global__ void k_bump_draw_epoch(view v)
 		v.draw_epoch[r]++;
 }
 
-__global__ void k_mark_divide(view v)
+// The phenotype update's visit of every agent, once: the moves the
+// compaction before it planned, the draws (the same as k_flag_by_draws),
+// the division list, and the removal test of the agents that do not divide
+// (k_divide_apply tests a parent and its daughter after it moved them).
+// One pass instead of five, of which three read the flags and two the
+// positions of all agents: bound by those bytes.
+template <int DIMS, bool DRAWS>
+__global__ void __launch_bounds__(kThreads) k_phenotype(view v, int cur, double p_divide, double p_death)
 {
 	grid_wait();
 	const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -3426,21 +3469,40 @@ __global__ void k_mark_divide(view v)
 	int r, local;
 	if (!live(v, s, r, local))
 		return;
-	if (v.flags[s] == PPC_FLAG_TO_DIVIDE)
+	if (DRAWS && *v.moves_pending != 0 && apply_move(v, cur, s))
+		v.move_src[s] = kMoved; // for the rebuild's count
+	const double4 p = v.pos[cur][s];
+	uint8_t flag = v.flags[s];
+	if (DRAWS)
 	{
-		int k = atomicAdd(&v.ctr[r].ndiv, 1);
+		const uint64_t ep = v.draw_epoch[r];
+		const uint8_t was = flag;
+		if (ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)local, PPC_DRAW_DEATH) < p_death)
+			flag = PPC_FLAG_TO_REMOVE;
+		else if (ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)local, PPC_DRAW_DIVIDE) < p_divide)
+			flag = PPC_FLAG_TO_DIVIDE;
+		if (flag != was)
+			v.flags[s] = flag;
+	}
+	if (flag == PPC_FLAG_TO_DIVIDE)
+	{
+		const int k = atomicAdd(&v.ctr[r].ndiv, 1);
 		if (k < v.reps[r].cap)
 			v.divl[v.reps[r].base + k] = local;
 		else
 			atomicOr(v.err, ERR_LIST_CAPACITY);
 	}
+	else if (to_remove<DIMS>(v.reps[r], p, flag))
+		append_bad(v, r, local);
 }
 
 // Orders the dividing agents (one block per replicate); daughters are
 // appended in ascending parent order like the serial reference loop. With
 // springs, thread 0 removes each parent from its partners' rows in that order
-// (cell::divide, reference: src/cell.cpp:110-114).
-__global__ void k_divide_plan(view v, int springs)
+// (cell::divide, reference: src/cell.cpp:110-114). `drawn`: the phenotype
+// draws used up an epoch.
+template <int DIMS>
+__global__ void k_divide_plan(view v, int cur, int springs, int drawn)
 {
 	grid_wait();
 	__shared__ int32_t sh[kSortCap];
@@ -3449,19 +3511,36 @@ __global__ void k_divide_plan(view v, int springs)
 	const int nd = min(C.ndiv, v.reps[r].cap);
 	const int base = v.reps[r].base;
 	if (threadIdx.x == 0)
+	{
 		C.nvisit = C.count;
+		if (drawn)
+			v.draw_epoch[r]++;
+	}
 	if (nd == 0)
 		return;
 	block_sort(v.divl + base, nd, sh);
-	if (threadIdx.x != 0)
-		return;
 	if (C.count + nd > v.reps[r].cap)
 	{
-		atomicOr(v.err, ERR_AGENT_CAPACITY);
-		C.ndiv = 0;
+		// nobody divides; the agents that would have are tested as they are
+		for (int k = threadIdx.x; k < nd; k += blockDim.x)
+		{
+			const int local = v.divl[base + k];
+			if (to_remove<DIMS>(v.reps[r], v.pos[cur][base + local], v.flags[base + local]))
+				append_bad(v, r, local);
+		}
+		__syncthreads();
+		if (threadIdx.x == 0)
+		{
+			atomicOr(v.err, ERR_AGENT_CAPACITY);
+			C.ndiv = 0;
+		}
 		return;
 	}
+	if (threadIdx.x != 0)
+		return;
 	*v.appended = 1; // daughters go past the count: the next k_bin_count takes new slots too
+	if (springs)
+		*v.params_changed = 1; // the partners' key-ordered rows carry their spring counts
 	if (springs)
 		for (int k = 0; k < nd; k++)
 		{
@@ -3487,7 +3566,10 @@ __global__ void k_divide_apply(view v, int cur)
 		const int p = base + lp;
 		const int c = base + n_pre + k;
 		v.flags[p] = PPC_FLAG_NONE;
-		*v.params_changed = 1; // the parent's radius and volumes change
+		// the parent's radius and volumes change, and the daughter may take a
+		// slot the last rebuild knew: the rebuild rewrites these two's copies
+		v.move_src[p] = v.move_src[c] = kMoved;
+		*v.moves_pending = 1;
 
 		// random direction, projected against the orientation by polarity and
 		// scaled by the parent's radius (reference: src/cell.cpp:129-150)
@@ -3579,21 +3661,11 @@ __global__ void k_divide_apply(view v, int cur)
 		}
 		v.pos[cur][p] = pp;
 		v.pos[cur][c] = pc;
+		if (to_remove<DIMS>(v.reps[r], pp, PPC_FLAG_NONE))
+			append_bad(v, r, lp);
+		if (to_remove<DIMS>(v.reps[r], pc, PPC_FLAG_NONE))
+			append_bad(v, r, n_pre + k);
 	}
-}
-
-__global__ void k_divide_finish(view v)
-{
-	grid_wait();
-	const int r = blockIdx.x * blockDim.x + threadIdx.x;
-	if (r >= v.nreps)
-		return;
-	rep_counters& C = v.ctr[r];
-	C.count += C.ndiv;
-	C.divisions += C.ndiv;
-	C.next_id += C.ndiv;
-	C.ndiv = 0;
-	v.draw_epoch[r]++;
 }
 
 // ---------------------------------------------------------------------------
@@ -4370,20 +4442,29 @@ int launch_mark_remove(ppc_state* s)
 	return PPC_OK;
 }
 
-int launch_divide(ppc_state* s)
+template <int DIMS>
+static void phenotype_dispatch(ppc_state* s, bool draws, double p_divide, double p_death)
 {
 	const int b = blocks_for(s->total_cap, kThreads);
 	const int springs = s->has_springs ? 1 : 0;
-	pdl(k_mark_divide, b, kThreads, 0, PPC_LAUNCH(s), s->v);
-	pdl(k_divide_plan, s->nreps, kThreads, 0, PPC_LAUNCH(s), s->v, springs);
+	auto k = draws ? k_phenotype<DIMS, true> : k_phenotype<DIMS, false>;
+	pdl(k, b, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur, p_divide, p_death);
+	pdl(k_divide_plan<DIMS>, s->nreps, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur, springs, draws ? 1 : 0);
 	dim3 g(std::max(1, std::min(64, blocks_for(s->total_cap / std::max(1, s->nreps), kThreads))), s->nreps);
+	pdl(k_divide_apply<DIMS>, g, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur);
+}
+
+// division and the removal candidates of the phenotype container update; with
+// `draws` after the moves of a folded compaction and the phenotype draws. The
+// compaction of the phenotype pass has to follow: it takes the daughters in.
+int launch_phenotype(ppc_state* s, bool draws, double p_divide, double p_death)
+{
 	if (s->dims == 1)
-		pdl(k_divide_apply<1>, g, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur);
+		phenotype_dispatch<1>(s, draws, p_divide, p_death);
 	else if (s->dims == 2)
-		pdl(k_divide_apply<2>, g, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur);
+		phenotype_dispatch<2>(s, draws, p_divide, p_death);
 	else
-		pdl(k_divide_apply<3>, g, kThreads, 0, PPC_LAUNCH(s), s->v, s->cur);
-	pdl(k_divide_finish, blocks_for(s->nreps, kThreads), kThreads, 0, PPC_LAUNCH(s), s->v);
+		phenotype_dispatch<3>(s, draws, p_divide, p_death);
 	PPC_CHECK_LAUNCH();
 	return PPC_OK;
 }
