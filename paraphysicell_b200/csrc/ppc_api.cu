@@ -690,27 +690,29 @@ int enqueue_step(ppc_state* s, bool phenotype, double p_divide, double p_death, 
 	return PPC_OK;
 }
 
-// one step through the separate entry points, for stochastic spring
-// attachment: the spring update needs every agent's neighbour list and its
-// attachments must be settled before the springs pull, so the step runs the
-// reference's sequence (simulator::simulate_mechanics, src/simulator.cpp:173-192)
-int enqueue_step_separate(ppc_state* s, bool phenotype, double p_divide, double p_death, bool last)
+// One step with stochastic spring attachment: the spring update needs every
+// agent's neighbours and its attachments must be settled before the springs
+// pull, so the step is a scan, the settlement, and the rest (the order of
+// simulator::simulate_mechanics, src/simulator.cpp:173-192, holds within each
+// agent's sums). 88,700 agents with every rate on: 114 us a step as the entry
+// points' kernels one after another, 83 us so.
+int enqueue_step_springs(ppc_state* s, bool phenotype, double p_divide, double p_death, bool last)
 {
-	PPC_TRY(launch_neighbors(s));
-	PPC_TRY(launch_forces(s));
-	if (s->params.virtual_wall_at_domain_edges)
-		PPC_TRY(launch_membrane(s));
-	PPC_TRY(launch_spring_updates(s));
-	PPC_TRY(launch_springs(s));
-	PPC_TRY(launch_positions(s));
-	PPC_TRY(launch_mark_remove(s));
-	PPC_TRY(launch_compact(s, false, true));
+	s->produce = !phenotype;
+	const int rc = launch_spring_step(s);
+	s->produce = false;
+	PPC_TRY(rc);
+	// the scan and k_spring_step read spring rows by slot, so only a call's
+	// last rebuild copies their counts into the key order
+	if (last)
+		PPC_TRY(mark_fields_changed(s));
+	PPC_TRY(launch_compact(s, false, true, !phenotype));
 	if (phenotype)
 	{
 		PPC_TRY(launch_phenotype(s, true, p_divide, p_death));
 		PPC_TRY(launch_compact(s, true, true));
 	}
-	PPC_TRY(launch_bin(s, false, last));
+	PPC_TRY(launch_bin(s, false, last, !phenotype));
 	return PPC_OK;
 }
 
@@ -872,7 +874,7 @@ int run_steps(ppc_state* s, int32_t steps, bool phenotype, double p_divide, doub
 		// non-zero attachment or detachment rates
 		s->has_springs = true;
 		for (int32_t k = 0; k < steps; k++)
-			PPC_TRY(enqueue_step_separate(s, phenotype, p_divide, p_death, k == steps - 1));
+			PPC_TRY(enqueue_step_springs(s, phenotype, p_divide, p_death, k == steps - 1));
 		s->lists_stale = steps > 0 || s->lists_stale;
 		return mark_ready(s);
 	}
@@ -1108,6 +1110,7 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 	a.want(v.tprev, (size_t)v.ntiles);
 	a.want(v.tdelta, (size_t)v.ntiles);
 	a.want(v.sdelta, ((size_t)v.ntiles + 1023) / 1024);
+	a.want(v.skeep, C);
 	a.want(v.chead, (size_t)v.ntiles * 32);
 	a.want(v.cnext, C);
 	a.want(v.porder, C);

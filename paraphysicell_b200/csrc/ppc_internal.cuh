@@ -163,6 +163,7 @@ struct view
 	int32_t* moves_pending; // a folded compaction left moves for them
 	int32_t* appended;		// agents were appended (division) since the last rebuild
 	uint8_t* sdel;		  // [C*S] spring marked for detachment this step
+	int32_t* skeep;		  // [C] spring row length without the marked ones
 	int32_t* first_end;	  // [C] INT32_MAX between spring attachment passes
 	int32_t* pos_changed; // set by an upload whose positions differ from the resident ones
 	int32_t* bin_active;  // the current rebuild runs (a conditional one may find nothing changed)
@@ -405,6 +406,8 @@ int launch_forces(ppc_state* s);
 int launch_membrane(ppc_state* s);
 int launch_springs(ppc_state* s);
 int launch_spring_updates(ppc_state* s);
+int launch_spring_step(ppc_state* s);
+int mark_fields_changed(ppc_state* s);
 int launch_positions(ppc_state* s);
 int launch_fused(ppc_state* s);
 int launch_step_persistent(ppc_state* s);
@@ -444,7 +447,6 @@ struct ix_fields
 	int32_t* order;	 // [n] the dependent agents still to walk, in index order
 };
 int launch_interactions(ppc_state* s, const ix_fields& x);
-int mark_fields_changed(ppc_state* s);
 
 // device copies of the ppc_motility fields of one replicate (local rows)
 struct mot_fields
