@@ -194,6 +194,22 @@ int finish(ppc_state* s)
 	return device_errors(s);
 }
 
+// finish, with the replicates' counts read in the same copy
+int finish_counts(ppc_state* s)
+{
+	PPC_CUDA(cudaGetLastError());
+	PPC_CUDA(cudaMemcpyAsync(s->pinned_ctr, s->v.ctr, sizeof(rep_counters) * (s->nreps + 1), cudaMemcpyDeviceToHost,
+							 s->stream)); // the counters and the error word
+	PPC_CUDA(cudaStreamSynchronize(s->stream));
+	for (int32_t k = 0; k < s->nreps; k++)
+		s->host_count[k] = s->pinned_ctr[k].count;
+	s->counts_known = true;
+	return PPC_OK;
+}
+
+// rows of a pass over replicate r whose kernels read the live count themselves
+int32_t most_rows(ppc_state* s, int32_t r) { return s->counts_known ? s->host_count[r] : s->reps[r].cap; }
+
 bool valid(ppc_state* s, int32_t r) { return s && r >= 0 && r < s->nreps; }
 
 int read_counters(ppc_state* s, std::vector<rep_counters>& c)
@@ -791,6 +807,8 @@ int replay_steps(ppc_state* s, int k, bool phenotype, double p_divide, double p_
 	s->vel_dirty = false;
 	return PPC_OK;
 }
+
+static_assert(sizeof(rep_counters) >= 4 * sizeof(int32_t), "the error word and three spare words end the counters");
 
 constexpr int kListLeast = 4;	   // steps of a call that run over lists
 constexpr int kListSteps = 100000; // steps of one launch over lists
@@ -1856,8 +1874,7 @@ int ppc_update_motility_fields(ppc_state* s, int32_t r, ppc_motility* f)
 		PPC_TRY(ppc_upload_motility(s, r, f)); // fields travel with the call
 	else if (!s->mot_store.p)
 		return fail(PPC_ERR_ARG, "no resident motility fields: upload them or pass fields");
-	int32_t n = 0;
-	PPC_TRY(live_count(s, r, n));
+	const int32_t n = most_rows(s, r); // known where the fields came with the call
 	if ((int32_t)s->mot_epoch.size() < s->nreps)
 		s->mot_epoch.resize(s->nreps, 0);
 	const uint64_t epoch = s->mot_epoch[r]++;
@@ -1906,7 +1923,8 @@ int ppc_update_motility_fields(ppc_state* s, int32_t r, ppc_motility* f)
 							 { { s->v.mot.vector, f->motility_vector, sizeof(double), (size_t)s->dims },
 							   { s->v.mot.direction, f->migration_bias_direction, sizeof(double), (size_t)s->dims } },
 							 s->reps[r].base, n, false));
-	return finish(s);
+	PPC_TRY(finish_counts(s));
+	return map_errors(s, *s->pinned_err);
 }
 
 int ppc_upload_gradients(ppc_state* s, int32_t r, const ppc_gradient_field* g)
@@ -1962,8 +1980,7 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 	}
 	else if (!s->ix_store.p)
 		return fail(PPC_ERR_ARG, "no resident interaction fields: upload them or pass fields");
-	int32_t n = 0;
-	PPC_TRY(live_count(s, r, n));
+	const int32_t n = most_rows(s, r); // known where the fields came with the call
 	if ((int32_t)s->ix_epoch.size() < s->nreps)
 		s->ix_epoch.resize(s->nreps, 0);
 	const uint64_t epoch = s->ix_epoch[r]++;
@@ -1971,7 +1988,7 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 		return PPC_OK;
 	PPC_TRY(ensure_lists(s));
 	const size_t nd = (size_t)n;
-	PPC_TRY(ensure_field_scratch(s, sizeof(int32_t) * (3 * nd + nd * s->ncap + 2)));
+	PPC_TRY(ensure_field_scratch(s, sizeof(int32_t) * (4 * nd + nd * s->ncap)));
 	int32_t* ip = static_cast<int32_t*>(s->ix_scratch);
 	const int32_t base = s->reps[r].base;
 	const ix_columns& c = s->v.ix;
@@ -1983,11 +2000,12 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 	x.base = base;
 	x.dt = s->params.mechanics_time_step;
 	x.epoch = epoch;
-	x.status = ip;
-	x.ncand = ip + 2;
-	x.dep = ip + 2 + nd;
-	x.cand = ip + 2 + 2 * nd;
-	x.order = ip + 2 + 2 * nd + nd * s->ncap;
+	x.status = s->v.err + 1; // the words after the error word, spare
+	x.ncand = ip;
+	x.dep = ip + nd;
+	x.walk = ip + 2 * nd;
+	x.order = ip + 3 * nd;
+	x.cand = ip + 4 * nd;
 	x.dead = c.dead + base;
 	x.dead_phago = c.dead_phago + base;
 	x.damage_rate = c.damage_rate + base;
@@ -2011,18 +2029,17 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 	x.target_cyto = c.target_cyto + base;
 	x.target_nuc = c.target_nuc + base;
 	x.isub = c.isub + base * S;
-	PPC_CUDA(cudaMemsetAsync(x.status, 0, 2 * sizeof(int32_t), s->stream));
+	PPC_CUDA(cudaMemsetAsync(x.status, 0, 3 * sizeof(int32_t), s->stream));
 	PPC_TRY(launch_interactions(s, x));
-	// the call's status and the device error word, with one synchronisation
-	PPC_CUDA(cudaMemcpyAsync(s->pinned_err + 1, x.status, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
-	PPC_CUDA(cudaMemcpyAsync(s->pinned_err, s->v.err, sizeof(int32_t), cudaMemcpyDeviceToHost, s->stream));
-	PPC_CUDA(cudaStreamSynchronize(s->stream));
-	PPC_CUDA(cudaGetLastError());
+	// the call's status, the device error word and the counts in one copy
+	PPC_TRY(finish_counts(s));
 	if (s->pinned_err[1])
 		return fail(PPC_ERR_CAPACITY, "a neighbour list exceeds the neighbour capacity: no interaction ran");
-	// positions and radii changed: the next mesh update rebuilds the bins; the
-	// neighbour lists stay those the interactions used, as in the reference
-	invalidate_bins(s);
+	// positions and radii may have changed: the next mesh update rebuilds the
+	// bins where they did (the device knows); the neighbour lists stay those
+	// the interactions used, as in the reference
+	s->bins_cond = s->bins_cond || s->bins_valid;
+	s->bins_valid = false;
 	if (f)
 	{
 		std::vector<column> back;

@@ -228,6 +228,8 @@ enum : int
 	LCTL_LEFT = 6	// steps a launch over lists left to the one behind it
 };
 
+constexpr int32_t kMoved = -2; // view::move_src: the slot's fields changed since the last rebuild
+
 struct buffer
 {
 	void* p = nullptr;
@@ -431,7 +433,8 @@ int launch_springs_local(ppc_state* s, int32_t r, int32_t n, int32_t* rows, int3
 // device copies of the ppc_interactions fields of one replicate (local rows)
 struct ix_fields
 {
-	int32_t n, substrates, replicate, base;
+	int32_t n; // rows at most; the device's count says how many
+	int32_t substrates, replicate, base;
 	double dt;
 	uint64_t epoch;
 	const uint8_t* dead;
@@ -442,16 +445,18 @@ struct ix_fields
 		*target_nuc, *isub;
 	int32_t* ncand; // [n] candidate neighbours of each agent
 	int32_t* cand;	// [n*ncap] their positions in the agent's neighbour list
-	int32_t* status; // [2] capacity error found by the candidate pass, count of agents left for the ordered pass
-	int32_t* dep;	 // [n] agents whose interactions depend on an earlier agent's
-	int32_t* order;	 // [n] the dependent agents still to walk, in index order
+	int32_t* status; // [3] capacity error found by the candidate pass, agents that walk, agents left for the ordered pass
+	int32_t* walk;	 // [n] the agents with a candidate
+	int32_t* dep;	 // [n] 1 while a dependent agent has not walked
+	int32_t* order;	 // [n] the dependent agents still to walk
 };
 int launch_interactions(ppc_state* s, const ix_fields& x);
 
 // device copies of the ppc_motility fields of one replicate (local rows)
 struct mot_fields
 {
-	int32_t n, replicate, base, per_agent, cur;
+	int32_t n; // rows at most; the device's count says how many
+	int32_t replicate, base, per_agent, cur;
 	double dt;
 	uint64_t epoch;
 	const uint8_t *motile, *restrict2d, *rule;

@@ -236,8 +236,6 @@ __device__ __forceinline__ int32_t voxel_key(const view& v, int cur, int s, int 
 // the slot's agent or its fields are not those of the last rebuild (a move
 // now or earlier, or kMoved left by the division): its key-ordered copies are
 // rewritten. A tail agent's own mark goes with it, and so never outlives it.
-constexpr int32_t kMoved = -2;
-
 __device__ __forceinline__ bool apply_move(const view& v, int cur, int s)
 {
 	const int src = v.move_src[s];

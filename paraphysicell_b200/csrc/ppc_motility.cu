@@ -88,7 +88,7 @@ template <int DIMS>
 __global__ void __launch_bounds__(kMotThreads) k_motility(view v, mot_fields m)
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
-	if (i >= m.n || m.motile[i] == 0)
+	if (i >= v.ctr[m.replicate].count || m.motile[i] == 0)
 		return;
 	double mv[DIMS];
 	for (int d = 0; d < DIMS; d++)
