@@ -74,6 +74,8 @@ struct rep_counters
 	int64_t deaths;		 // environment::deaths_count
 	int64_t next_id;	 // id of the next created agent
 	int32_t nattach;	 // entries in the spring-attachment candidate list
+	int32_t nrest;		 // of them, left for the last block of the settlement
+	int32_t attach_blocks; // blocks of the settlement that are through with theirs
 	int32_t pad;
 	int64_t spring_epoch; // spring updates so far: epoch of their counter-based draws
 };
@@ -336,6 +338,11 @@ struct ppc_state
 	size_t stage_used = 0; // bytes of the arena taken by the current transfer call
 	std::vector<ppc::pending_unpack> pending_unpacks;
 	std::vector<ppc::pending_copy> pending_copies;
+	// large copies to pageable host rows: their page-locked landing area and
+	// the host copies due once they have landed
+	void* bounce = nullptr;
+	size_t bounce_bytes = 0, bounce_used = 0;
+	std::vector<ppc::pending_copy> pending_host;
 
 	// captured CUDA graphs of blocks of fused steps (ppc_api.cu: replay_steps)
 	std::vector<ppc::graph_entry> graphs;
@@ -426,7 +433,7 @@ int launch_count_flags(ppc_state* s, int32_t r, int32_t flag, int32_t* count);
 int launch_unpack_vec(ppc_state* s, double4* dst, const double* src, int32_t r, int32_t n, int32_t* changed = nullptr);
 int launch_pack_vec(ppc_state* s, double* dst, const double4* src, int32_t r, int32_t n);
 int launch_unpack_prm(ppc_state* s, int field, const double* src, int32_t r, int32_t n);
-int launch_pack_prm(ppc_state* s, int field, double* dst, int32_t r, int32_t n);
+int launch_pack_prm(ppc_state* s, int field, double* dst, int32_t first, int32_t n);
 int launch_neighbors_local(ppc_state* s, int32_t r, int32_t n, int32_t* counts, int32_t* lists, int32_t cap);
 int launch_springs_local(ppc_state* s, int32_t r, int32_t n, int32_t* rows, int32_t cap, int to_device);
 
