@@ -2226,7 +2226,13 @@ __device__ __forceinline__ void attach_draws(const view& v, int r, int s, int j,
 	{
 		const int q = atomicAdd(&v.ctr[r].nattach, 1);
 		if (q < v.reps[r].cap)
-			v.divl[base + q] = li * v.ncap + k;
+		{
+			// the lowest code that names each agent, for k_spring_attach_apply
+			const int code = li * v.ncap + k;
+			v.divl[base + q] = code;
+			atomicMin(v.first_end + s, code);
+			atomicMin(v.first_end + j, code);
+		}
 		else
 			atomicOr(v.err, ERR_LIST_CAPACITY);
 	}
@@ -3291,15 +3297,18 @@ __global__ void k_spring_attach_draws(view v)
 		attach_draws(v, r, s, v.nidx[(int64_t)s * v.ncap + k], k);
 }
 
-// One block per replicate: the candidates in the reference's order (agent,
-// then neighbour position), attached while both rows are below their
-// maximum_number_of_attachments; then the replicate's spring epoch advances.
-// Up to kAttachCap candidates the block stages them in shared memory: each
-// endpoint's agent, maximum and row length, and the first endpoint of the
-// list that names the same agent (found with a per-slot atomicMin), whose
-// count slot all its endpoints share; the candidates then settle in waves
-// that touch only shared memory apart from the row writes. Longer lists take
-// the serial pass over global memory.
+// The candidates in the reference's order (agent, then neighbour position),
+// attached while both rows are below their maximum_number_of_attachments;
+// then the replicate's spring epoch advances. A candidate that is the lowest
+// one at both its agents sees the rows the serial loop would show it, so all
+// of these settle at once, over several blocks. The replicate's last block to
+// get there settles the rest: up to kAttachCap of them it stages in shared
+// memory, each endpoint's agent, maximum and row length, and the first
+// endpoint of the list that names the same agent (found with a per-slot
+// atomicMin), whose count slot all its endpoints share; they then settle in
+// waves that touch only shared memory apart from the row writes. Longer lists
+// take the serial pass over global memory. 88,700 agents, some 2,700
+// candidates a step: 30 us with all of them in one block, 22 us so (cold caches).
 constexpr int kAttachCap = 4096;
 constexpr int kAttachThreads = 1024;
 constexpr int kAttachWaves = 32;	 // parallel waves at most before the remaining candidates go in order
@@ -3362,7 +3371,7 @@ __device__ __forceinline__ void attach_settle(const view& v, const int32_t* agen
 	cnt[rj] = nj + 1;
 }
 
-__global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v)
+__global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v, int parts)
 {
 	grid_wait();
 	extern __shared__ int32_t dyn[];
@@ -3373,11 +3382,51 @@ __global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v)
 	int16_t* mx = reinterpret_cast<int16_t*>(low + 2 * kAttachCap); // [2 cap] maximum_number_of_attachments
 	int16_t* rep = mx + 2 * kAttachCap;		   // [2 cap] first endpoint naming the same agent
 	uint8_t* done = reinterpret_cast<uint8_t*>(rep + 2 * kAttachCap); // [cap] settled
-	const int r = blockIdx.x;
+	const int r = blockIdx.x / parts, part = blockIdx.x % parts;
 	rep_counters& C = v.ctr[r];
 	const int base = v.reps[r].base;
-	const int nc = min(C.nattach, v.reps[r].cap);
-	int32_t* codes = v.divl + base;
+	const int listed = min(C.nattach, v.reps[r].cap);
+	int32_t* codes = v.moves + 2 * (int64_t)base; // the candidates left (no moves are planned at this time)
+	for (int q = part * blockDim.x + threadIdx.x; q < listed; q += parts * blockDim.x)
+	{
+		const int code = v.divl[base + q];
+		const int i = base + code / v.ncap;
+		const int j = v.nidx[(int64_t)i * v.ncap + code % v.ncap];
+		const bool low_i = __ldcg(v.first_end + i) == code, low_j = __ldcg(v.first_end + j) == code;
+		if (low_i && low_j)
+		{
+			const int ni = __ldcg(v.scnt + i), nj = __ldcg(v.scnt + j);
+			if (ni < v.maxatt[i] && nj < v.maxatt[j])
+			{
+				if (ni >= v.scap || nj >= v.scap)
+					atomicOr(v.err, ERR_SPRING_CAPACITY);
+				else
+				{
+					v.springs[(int64_t)i * v.scap + ni] = j;
+					v.springs[(int64_t)j * v.scap + nj] = i;
+					v.scnt[i] = ni + 1;
+					v.scnt[j] = nj + 1;
+				}
+			}
+		}
+		else
+			codes[atomicAdd(&C.nrest, 1)] = code;
+		// each agent's word is restored by the candidate it names
+		if (low_i)
+			v.first_end[i] = INT32_MAX;
+		if (low_j)
+			v.first_end[j] = INT32_MAX;
+	}
+	__shared__ int s_last;
+	__threadfence();
+	__syncthreads();
+	if (threadIdx.x == 0)
+		s_last = atomicAdd(&C.attach_blocks, 1) == parts - 1;
+	__syncthreads();
+	if (!s_last)
+		return;
+	__threadfence();
+	const int nc = __ldcg(&C.nrest);
 	if (nc <= kAttachCap)
 	{
 		// The candidates stay in the order the draws listed them: the
@@ -3392,7 +3441,7 @@ __global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v)
 			for (int k = 0; k < kAttachBatch; k++)
 			{
 				const int q = q0 + k * blockDim.x;
-				code[k] = q < nc ? codes[q] : -1;
+				code[k] = q < nc ? __ldcg(codes + q) : -1;
 			}
 #pragma unroll
 			for (int k = 0; k < kAttachBatch; k++)
@@ -3405,8 +3454,8 @@ __global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v)
 			for (int k = 0; k < kAttachBatch; k++)
 			{
 				const bool ok = code[k] >= 0;
-				ci[k] = ok ? v.scnt[ii[k]] : 0;
-				cj[k] = ok ? v.scnt[jj[k]] : 0;
+				ci[k] = ok ? __ldcg(v.scnt + ii[k]) : 0;
+				cj[k] = ok ? __ldcg(v.scnt + jj[k]) : 0;
 				mi[k] = ok ? v.maxatt[ii[k]] : 0;
 				mj[k] = ok ? v.maxatt[jj[k]] : 0;
 			}
@@ -3528,7 +3577,7 @@ __global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v)
 				const int code = codes[q];
 				const int i = base + code / v.ncap;
 				const int j = v.nidx[(int64_t)i * v.ncap + code % v.ncap];
-				const int ni = v.scnt[i], nj = v.scnt[j];
+				const int ni = __ldcg(v.scnt + i), nj = __ldcg(v.scnt + j);
 				if (ni < v.maxatt[i] && nj < v.maxatt[j])
 				{
 					if (ni >= v.scap || nj >= v.scap)
@@ -3545,7 +3594,7 @@ __global__ void __launch_bounds__(kAttachThreads) k_spring_attach_apply(view v)
 	}
 	if (threadIdx.x == 0)
 	{
-		C.nattach = 0;
+		C.nattach = C.nrest = C.attach_blocks = 0;
 		C.spring_epoch++;
 	}
 }
@@ -4171,6 +4220,13 @@ int mark_fields_changed(ppc_state* s)
 	return PPC_OK;
 }
 
+// blocks per replicate that share out the attachment candidates: a block for
+// some 8,192 agents, whose candidates are a few hundred
+static int attach_parts(ppc_state* s)
+{
+	return std::max(1, std::min(32, s->total_cap / std::max(1, s->nreps) / 8192));
+}
+
 template <int DIMS>
 static int spring_step_dispatch(ppc_state* s)
 {
@@ -4182,7 +4238,8 @@ static int spring_step_dispatch(ppc_state* s)
 	pdl(k_spring_scan<DIMS>, b, kQueueThreads, dyn, PPC_LAUNCH(s), s->v, s->cur, (int)FUSED_VEL);
 	PPC_CUDA(cudaFuncSetAttribute(k_spring_attach_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
 								  (int)kAttachSmem));
-	pdl(k_spring_attach_apply, s->nreps, kAttachThreads, kAttachSmem, PPC_LAUNCH(s), s->v);
+	pdl(k_spring_attach_apply, s->nreps * attach_parts(s), kAttachThreads, kAttachSmem, PPC_LAUNCH(s), s->v,
+		attach_parts(s));
 	pdl(k_spring_step<DIMS>, b, kQueueThreads, 0, PPC_LAUNCH(s), s->v, s->cur,
 		walls | FUSED_VEL | (s->produce ? FUSED_PRODUCE : 0));
 	PPC_CHECK_LAUNCH();
@@ -4208,7 +4265,8 @@ int launch_spring_updates(ppc_state* s)
 	pdl(k_spring_attach_draws, b, kThreads, 0, PPC_LAUNCH(s), s->v);
 	PPC_CUDA(cudaFuncSetAttribute(k_spring_attach_apply, cudaFuncAttributeMaxDynamicSharedMemorySize,
 								  (int)kAttachSmem));
-	pdl(k_spring_attach_apply, s->nreps, kAttachThreads, kAttachSmem, PPC_LAUNCH(s), s->v);
+	pdl(k_spring_attach_apply, s->nreps * attach_parts(s), kAttachThreads, kAttachSmem, PPC_LAUNCH(s), s->v,
+		attach_parts(s));
 	PPC_CHECK_LAUNCH();
 	return PPC_OK;
 }
@@ -4677,11 +4735,11 @@ int launch_unpack_prm(ppc_state* s, int field, const double* src, int32_t r, int
 	return PPC_OK;
 }
 
-int launch_pack_prm(ppc_state* s, int field, double* dst, int32_t r, int32_t n)
+int launch_pack_prm(ppc_state* s, int field, double* dst, int32_t first, int32_t n)
 {
 	if (n == 0)
 		return PPC_OK;
-	pdl(k_pack_prm, blocks_for(n, kThreads), kThreads, 0, PPC_LAUNCH(s), s->v, field, dst, s->reps[r].base, n);
+	pdl(k_pack_prm, blocks_for(n, kThreads), kThreads, 0, PPC_LAUNCH(s), s->v, field, dst, first, n);
 	PPC_CHECK_LAUNCH();
 	return PPC_OK;
 }
