@@ -2252,9 +2252,16 @@ __device__ __forceinline__ void compact_springs(const view& v, int s)
 
 // Evaluates the warp's kept candidates [0, nh) in rounds of 32 and adds each
 // agent's terms to its sums in list order. LISTS: they also go to the
-// neighbour list of the agent (slot s, nn neighbours so far) with their
-// attachment draws.
-template <int DIMS, bool F32, bool LISTS>
+// neighbour list of the agent (slot s, nn neighbours so far), with their
+// attachment draws or (LISTS_ONLY) without draws and sums.
+enum : int
+{
+	LISTS_NONE = 0,
+	LISTS_DRAWS = 1,
+	LISTS_ONLY = 2
+};
+
+template <int DIMS, bool F32, int LISTS>
 __device__ __forceinline__ void queue_hits(const view& v, queue_warp& w, int nh, bool act, bool mov_i, double& vx,
 										   double& vy, double& vz, double& pressure, nsum& fx, nsum& fy, nsum& fz,
 										   nsum& fp, int r, int s, int& nn)
@@ -2291,7 +2298,9 @@ __device__ __forceinline__ void queue_hits(const view& v, queue_warp& w, int nh,
 				d2 = d2 + ddz * ddz;
 			const double ad = pa.w + q.w;
 			const double dist = DIMS == 1 ? fabs(ddx) : sqrt(d2);
-			if (F32)
+			if (LISTS == LISTS_ONLY)
+				flags = dist <= ad ? 1 : 0;
+			else if (F32)
 			{
 				// pair_fp32::add with the agent's values
 				const float4 qj = v.sprmf[u];
@@ -2357,10 +2366,13 @@ __device__ __forceinline__ void queue_hits(const view& v, queue_warp& w, int nh,
 				}
 			}
 		}
-		w.term[lane] = term;
-		w.fx[lane] = tx;
-		w.fy[lane] = ty;
-		w.fz[lane] = tz;
+		if (LISTS != LISTS_ONLY)
+		{
+			w.term[lane] = term;
+			w.fx[lane] = tx;
+			w.fy[lane] = ty;
+			w.fz[lane] = tz;
+		}
 		w.hflags[lane] = flags;
 		const unsigned grp = __match_any_sync(0xffffffffu, own);
 		if (own >= 0 && lane == __ffs(grp) - 1)
@@ -2383,10 +2395,13 @@ __device__ __forceinline__ void queue_hits(const view& v, queue_warp& w, int nh,
 					if (nn < v.ncap)
 					{
 						v.nidx[(int64_t)s * v.ncap + nn] = j;
-						attach_draws(v, r, s, j, nn);
+						if (LISTS == LISTS_DRAWS)
+							attach_draws(v, r, s, j, nn);
 					}
 					nn++;
 				}
+				if (LISTS == LISTS_ONLY)
+					continue;
 				const double tm = w.term[l];
 				if (F32)
 				{
@@ -2421,11 +2436,12 @@ __device__ __forceinline__ void queue_hits(const view& v, queue_warp& w, int nh,
 }
 
 // The agent at key-ordered position t; every lane of the warp calls it.
-// LISTS: the first half of a step with stochastic springs. It makes the
+// LISTS_DRAWS: the first half of a step with stochastic springs. It makes the
 // neighbour lists, the attachment draws and the pair sums in one scan, and
 // drops the springs k_spring_detach marked; the sums stay in vel and pressure
 // for k_spring_step, which runs once the attachments are settled.
-template <int DIMS, bool F32, bool LISTS = false>
+// LISTS_ONLY: the neighbour lists.
+template <int DIMS, bool F32, int LISTS = LISTS_NONE>
 __device__ __forceinline__ void fused_queue_agent(const view& v, int cur, int opts, int t, queue_warp& w)
 {
 	constexpr int NR = DIMS == 3 ? 9 : (DIMS == 2 ? 3 : 1);
@@ -2459,7 +2475,7 @@ __device__ __forceinline__ void fused_queue_agent(const view& v, int cur, int op
 	const rep_info& R = v.reps[r];
 	const int D = v.ndefs;
 	int lo[NR], hi[NR];
-	if (act)
+	if (act && (LISTS != LISTS_ONLY || mov_i)) // an agent that does not move has no list
 	{
 		// this agent's affinity row: read per neighbour by definition index
 		if (F32)
@@ -2494,7 +2510,7 @@ __device__ __forceinline__ void fused_queue_agent(const view& v, int cur, int op
 	// now, with the first two spring partners' rows once their indices arrive
 	const int nspr = (act && springs_on && mov_i) ? unpack_springs(qi.w) : 0;
 	int j0 = -1, j1 = -1;
-	if (act)
+	if (act && LISTS != LISTS_ONLY)
 	{
 		prefetch_l2(v.flags + s);
 		if (mov_i)
@@ -2627,10 +2643,12 @@ __device__ __forceinline__ void fused_queue_agent(const view& v, int cur, int op
 	}
 	if (LISTS)
 	{
-		compact_springs(v, s);
 		v.ncnt[s] = nn;
 		if (nn > v.ncap)
 			atomicOr(v.err, ERR_NEIGHBOR_CAPACITY);
+		if (LISTS == LISTS_ONLY)
+			return;
+		compact_springs(v, s);
 		v.pressure[s] = pressure;
 		if (mov_i)
 			v.vel[s] = make_double4(vx, vy, vz, 0.0);
@@ -2665,7 +2683,7 @@ __global__ void __launch_bounds__(kQueueThreads, 5) k_spring_scan(view v, int cu
 	grid_wait();
 	extern __shared__ __align__(16) unsigned char queue_raw[];
 	queue_smem& sm = *reinterpret_cast<queue_smem*>(queue_raw);
-	fused_queue_agent<DIMS, false, true>(v, cur, opts, blockIdx.x * kQueueThreads + threadIdx.x,
+	fused_queue_agent<DIMS, false, LISTS_DRAWS>(v, cur, opts, blockIdx.x * kQueueThreads + threadIdx.x,
 										 sm.w[threadIdx.x >> 5]);
 }
 
@@ -2693,33 +2711,18 @@ __global__ void __launch_bounds__(kQueueThreads) k_spring_step(view v, int cur, 
 // separate reference entry points
 // ---------------------------------------------------------------------------
 
-// position_solver::update_cell_neighbors (reference: position_solver.cpp:262-286)
+// position_solver::update_cell_neighbors (reference: position_solver.cpp:262-286):
+// the scan of k_fused_queue, whose warps share out their candidates. 20,011
+// agents: 23.5 us with a thread per agent walking its own, 19 us so
+// (cold caches).
 template <int DIMS>
-__global__ void __launch_bounds__(kThreads) k_neighbors(view v)
+__global__ void __launch_bounds__(kQueueThreads, 5) k_neighbors(view v)
 {
 	grid_wait();
-	const int t = blockIdx.x * blockDim.x + threadIdx.x;
-	if (t >= *v.cursor)
-		return;
-	const int s = v.sorted[t];
-	if (v.movable[s] == 0)
-	{
-		v.ncnt[s] = 0;
-		return;
-	}
-	const rep_info& R = v.reps[rep_of(v, s)];
-	int n = 0;
-	int32_t* out = v.nidx + (int64_t)s * v.ncap;
-	const int cap = v.ncap;
-	__shared__ int32_t list[kList * kThreads];
-	for_each_neighbor<DIMS>(v, R, t, v.skey[t], v.spos4[t], list + threadIdx.x, [&](int u) {
-		if (n < cap)
-			out[n] = v.sorted[u];
-		n++;
-	});
-	if (n > cap)
-		atomicOr(v.err, ERR_NEIGHBOR_CAPACITY);
-	v.ncnt[s] = n;
+	extern __shared__ __align__(16) unsigned char queue_raw[];
+	queue_smem& sm = *reinterpret_cast<queue_smem*>(queue_raw);
+	fused_queue_agent<DIMS, false, LISTS_ONLY>(v, 0, 0, blockIdx.x * kQueueThreads + threadIdx.x,
+											   sm.w[threadIdx.x >> 5]);
 }
 
 __global__ void k_clear_pressure(view v)
@@ -4160,13 +4163,10 @@ int launch_bin(ppc_state* s, bool conditional, bool ready, bool produced)
 
 int launch_neighbors(ppc_state* s)
 {
-	const int b = blocks_for(s->total_cap, kThreads);
-	if (s->dims == 1)
-		pdl(k_neighbors<1>, b, kThreads, 0, PPC_LAUNCH(s), s->v);
-	else if (s->dims == 2)
-		pdl(k_neighbors<2>, b, kThreads, 0, PPC_LAUNCH(s), s->v);
-	else
-		pdl(k_neighbors<3>, b, kThreads, 0, PPC_LAUNCH(s), s->v);
+	const int dyn = (int)sizeof(queue_smem);
+	auto k = s->dims == 1 ? k_neighbors<1> : (s->dims == 2 ? k_neighbors<2> : k_neighbors<3>);
+	PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn));
+	pdl(k, blocks_for(s->total_cap, kQueueThreads), kQueueThreads, dyn, PPC_LAUNCH(s), s->v);
 	PPC_CHECK_LAUNCH();
 	return PPC_OK;
 }
