@@ -183,7 +183,7 @@ void drain_host(ppc_state* s)
 // memory with one thread, 5.5 GB/s; a large copy lands in the state's
 // page-locked area instead and drain_host, after the next synchronisation,
 // spreads the host copy over a few threads. 1 M agents, 72 MB of them 16 MB
-// pageable: 4.0 and 2.5 ms (of it: agents appended since the
+// pageable: 4.0 and 2.1 ms (of it: agents appended since the
 // last count no longer cost a second download of all).
 int copy_down(ppc_state* s, void* dst, const void* src, size_t bytes)
 {
@@ -207,6 +207,7 @@ int copy_down(ppc_state* s, void* dst, const void* src, size_t bytes)
 		char* land = static_cast<char*>(s->bounce) + s->bounce_used;
 		PPC_CUDA(cudaMemcpyAsync(land, src, n, cudaMemcpyDeviceToHost, s->stream));
 		s->pending_host.push_back({ dst, land, n });
+		s->bounce_pieces++;
 		s->bounce_used += n;
 		dst = static_cast<char*>(dst) + n;
 		src = static_cast<const char*>(src) + n;
@@ -633,7 +634,7 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 }
 
 // queues the copies of agents [first, n) of replicate r into the host view
-// (no synchronisation)
+// (large pageable columns are waited for, the rest is not)
 int copy_out(ppc_state* s, int32_t r, ppc_agents* a, int32_t first, int32_t n)
 {
 	const int32_t base = s->reps[r].base;
@@ -643,7 +644,6 @@ int copy_out(ppc_state* s, int32_t r, ppc_agents* a, int32_t first, int32_t n)
 	PPC_TRY(get_vec(s, a->velocities, v.vel, r, first, n));
 	PPC_TRY(get_vec(s, a->previous_velocities, v.vprev, r, first, n));
 	PPC_TRY(get_vec(s, a->orientation, v.orient, r, first, n));
-	PPC_TRY(flush_copies(s));
 	PPC_TRY(get_prm(s, 0, a->radius, r, first, n));
 	PPC_TRY(get_prm(s, 1, a->cell_cell_repulsion_strength, r, first, n));
 	PPC_TRY(get_prm(s, 2, a->cell_cell_adhesion_strength, r, first, n));
@@ -664,6 +664,18 @@ int copy_out(ppc_state* s, int32_t r, ppc_agents* a, int32_t first, int32_t n)
 	PPC_TRY(get_scalar(s, a->is_movable, v.movable, base, first, n, 1));
 	PPC_TRY(get_scalar(s, a->flags, v.flags, base, first, n, 1));
 	PPC_TRY(get_scalar(s, a->agent_ids, v.ids, base, first, n, 1));
+	// the vectors' copies last, so that the host copies of the columns that
+	// landed before them run beside these
+	const uint64_t pieces = s->bounce_pieces;
+	const bool landing = !s->pending_host.empty();
+	if (landing)
+		PPC_CUDA(cudaEventRecord(s->ev_landed, s->stream));
+	PPC_TRY(flush_copies(s));
+	if (landing && s->bounce_pieces == pieces) // page-locked vectors: none of them uses the landing area
+	{
+		PPC_CUDA(cudaEventSynchronize(s->ev_landed));
+		drain_host(s);
+	}
 	return PPC_OK;
 }
 
@@ -1161,7 +1173,8 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 			|| cudaEventCreateWithFlags(&s->ev_h2d, cudaEventDisableTiming) != cudaSuccess
 			|| cudaEventCreateWithFlags(&s->ev_stage_free, cudaEventDisableTiming) != cudaSuccess
 			|| cudaEventCreateWithFlags(&s->ev_fork, cudaEventDisableTiming) != cudaSuccess
-			|| cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming) != cudaSuccess))
+			|| cudaEventCreateWithFlags(&s->ev_join, cudaEventDisableTiming) != cudaSuccess
+			|| cudaEventCreateWithFlags(&s->ev_landed, cudaEventDisableTiming) != cudaSuccess))
 		rc = fail(PPC_ERR_CUDA, "cudaStreamCreate or cudaEventCreate failed");
 
 	view& v = s->v;
@@ -1342,7 +1355,7 @@ int ppc_destroy(ppc_state* s)
 	release_graph(s);
 	for (auto e : s->prof_events)
 		cudaEventDestroy(e);
-	for (auto e : { s->ev_ready, s->ev_h2d, s->ev_stage_free, s->ev_fork, s->ev_join })
+	for (auto e : { s->ev_ready, s->ev_h2d, s->ev_stage_free, s->ev_fork, s->ev_join, s->ev_landed })
 		if (e)
 			cudaEventDestroy(e);
 	if (s->xfer)

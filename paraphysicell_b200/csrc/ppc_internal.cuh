@@ -297,7 +297,8 @@ struct ppc_state
 	// of the rebuild.
 	cudaStream_t xfer = nullptr;
 	cudaStream_t h2d_stream = nullptr; // the stream an upload's host copies go to (null: `stream`)
-	cudaEvent_t ev_ready = nullptr, ev_h2d = nullptr, ev_stage_free = nullptr, ev_fork = nullptr, ev_join = nullptr;
+	cudaEvent_t ev_ready = nullptr, ev_h2d = nullptr, ev_stage_free = nullptr, ev_fork = nullptr, ev_join = nullptr,
+				ev_landed = nullptr;
 	bool join_pending = false; // a capture forked the transfer stream for ev_ready
 	bool ready_pending = false;	 // ev_ready marks the state a download reads...
 	int64_t ready_launches = 0;	 // ...while no kernel has been launched since (launch count then)
@@ -342,6 +343,7 @@ struct ppc_state
 	// the host copies due once they have landed
 	void* bounce = nullptr;
 	size_t bounce_bytes = 0, bounce_used = 0;
+	uint64_t bounce_pieces = 0; // copies into it so far
 	std::vector<ppc::pending_copy> pending_host;
 
 	// captured CUDA graphs of blocks of fused steps (ppc_api.cu: replay_steps)
