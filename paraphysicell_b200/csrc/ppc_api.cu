@@ -135,6 +135,8 @@ int flush_unpacks(ppc_state* s)
 	return PPC_OK;
 }
 
+const void* mapped(const void* host);
+
 constexpr size_t kBounceMost = (size_t)32 << 20; // page-locked bytes of a state's landing area
 constexpr size_t kBounceLeast = (size_t)1 << 20; // smaller copies are left to the driver
 constexpr int kHostThreads = 4;
@@ -177,6 +179,24 @@ void drain_host(ppc_state* s)
 			t.join();
 	s->pending_host.clear();
 	s->bounce_used = 0;
+}
+
+// Rows up to this size go between mapped host rows and the device by kernels,
+// which cost less than copies' latency: a download's columns in one launch.
+constexpr size_t kSmallRows = 64 * 1024;
+
+// takes a column of a small download into the launch that follows; false where
+// it has to be copied
+bool pull_column(ppc_state* s, void* dst, const void* src, size_t bytes, int width)
+{
+	if (!s->pulling || bytes > kSmallRows || bytes % 4 || (reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) % (width ? 8 : 4)
+		|| s->pull.count == pull_list::kMost)
+		return false;
+	void* d = const_cast<void*>(mapped(dst));
+	if (!d)
+		return false;
+	s->pull.job[s->pull.count++] = { d, src, (int32_t)(bytes / (width ? 8 : 4)), width };
+	return true;
 }
 
 // Queues a device-to-host copy on the stream. The driver copies into pageable
@@ -340,7 +360,9 @@ int put_scalar(ppc_state* s, T* dev, const T* host, int32_t base, int32_t n, siz
 template <typename T>
 int get_scalar(ppc_state* s, T* host, const T* dev, int32_t base, int32_t first, int32_t n, size_t width)
 {
-	if (host && n > first)
+	if (host && n > first
+		&& !pull_column(s, host + (size_t)first * width, dev + (size_t)(base + first) * width,
+						(size_t)(n - first) * width * sizeof(T), 0))
 		PPC_TRY(copy_down(s, host + (size_t)first * width, dev + (size_t)(base + first) * width,
 						  (size_t)(n - first) * width * sizeof(T)));
 	return PPC_OK;
@@ -370,7 +392,7 @@ int put_vec(ppc_state* s, double4* dev, const double* host, int32_t r, int32_t n
 		return PPC_OK;
 	if (n == 0)
 		return PPC_OK;
-	if (host && s->zero_copy)
+	if (host && (s->zero_copy || s->direct_rows))
 		if (const void* d = mapped(host))
 			return launch_unpack_vec(s, dev, static_cast<const double*>(d), r, n, changed);
 	const size_t bytes = (size_t)n * s->dims * sizeof(double);
@@ -393,6 +415,8 @@ int get_vec(ppc_state* s, double* host, const double4* dev, int32_t r, int32_t f
 	host += (size_t)first * s->dims;
 	dev += first;
 	n -= first;
+	if (pull_column(s, host, dev + s->reps[r].base, (size_t)n * s->dims * sizeof(double), s->dims))
+		return PPC_OK;
 	if (s->zero_copy)
 		if (const void* d = mapped(host))
 			return launch_pack_vec(s, static_cast<double*>(const_cast<void*>(d)), dev, r, n);
@@ -500,7 +524,9 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 	// transfer stream, beside whatever the stream still runs (the last step's
 	// mesh rebuild); the arena is free once the stream has unpacked the
 	// previous upload, and the unpacks wait for the copies
-	const bool beside = kinematic && pinned && !s->zero_copy && s->xfer;
+	const bool small = kinematic && pinned && (size_t)n * s->dims * sizeof(double) <= kSmallRows;
+	const bool beside = kinematic && pinned && !small && !s->zero_copy && s->xfer;
+	s->direct_rows = small;
 	if (beside)
 	{
 		PPC_CUDA(cudaStreamWaitEvent(s->xfer, s->ev_stage_free, 0));
@@ -514,6 +540,7 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 	if (rc == PPC_OK)
 		rc = put_vec(s, v.orient, a->orientation, r, n, defaults);
 	s->h2d_stream = nullptr;
+	s->direct_rows = false;
 	PPC_TRY(rc);
 	if (beside)
 	{
@@ -688,9 +715,15 @@ int transfer_out_on(ppc_state* s, int32_t r, ppc_agents* a, cudaStream_t main, b
 	// previous count, within the host capacity, may be overwritten.
 	stage_reset(s);
 	const int32_t guess = std::max(0, std::min(s->host_count[r], std::min(a->capacity, s->reps[r].cap)));
-	PPC_CUDA(cudaMemcpyAsync(s->pinned_ctr, s->v.ctr, sizeof(rep_counters) * (s->nreps + 1), cudaMemcpyDeviceToHost,
-							 s->stream)); // the counters and the error word
-	PPC_TRY(copy_out(s, r, a, 0, guess));
+	s->pull.count = 0;
+	s->pulling = (size_t)guess * s->dims * sizeof(double) <= kSmallRows;
+	const size_t head = sizeof(rep_counters) * (s->nreps + 1); // the counters and the error word
+	if (!pull_column(s, s->pinned_ctr, s->v.ctr, head, 0))
+		PPC_CUDA(cudaMemcpyAsync(s->pinned_ctr, s->v.ctr, head, cudaMemcpyDeviceToHost, s->stream));
+	const int rc = copy_out(s, r, a, 0, guess);
+	s->pulling = false;
+	PPC_TRY(rc);
+	PPC_TRY(launch_pull(s));
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
 	drain_host(s);
 	if (beside && *s->pinned_err)

@@ -262,6 +262,22 @@ struct pending_copy
 	size_t bytes;
 };
 
+// a column of a small download: `n` 4-byte words (width 0) or doubles, `width`
+// of each four of the device rows, into mapped host rows
+struct pull_job
+{
+	void* dst;
+	const void* src;
+	int32_t n, width;
+};
+
+struct pull_list
+{
+	static constexpr int kMost = 16;
+	pull_job job[kMost];
+	int32_t count = 0;
+};
+
 // one captured block of fused steps and what its kernels were captured with
 struct graph_entry
 {
@@ -315,6 +331,7 @@ struct ppc_state
 	bool bins_valid = false;	  // bins match the current positions
 	bool bins_cond = false;		  // ...unless an upload changed them: the device decides (pos_changed)
 	bool counts_known = false;	  // host_count holds the device counts (no count-changing work since)
+	bool direct_rows = false;	  // the same for the rows of the upload being queued, which are few
 	bool zero_copy = false;		  // pinned host rows are read and written by kernels over the bus
 	bool lists_stale = false;	  // a fused step ran since the neighbour lists were built
 	// the lists that outlive a step: whether they and their key-ordered copies
@@ -343,6 +360,8 @@ struct ppc_state
 	// the host copies due once they have landed
 	void* bounce = nullptr;
 	size_t bounce_bytes = 0, bounce_used = 0;
+	ppc::pull_list pull; // jobs of the small download being queued
+	bool pulling = false;
 	uint64_t bounce_pieces = 0; // copies into it so far
 	std::vector<ppc::pending_copy> pending_host;
 
@@ -435,6 +454,7 @@ int launch_count_flags(ppc_state* s, int32_t r, int32_t flag, int32_t* count);
 int launch_unpack_vec(ppc_state* s, double4* dst, const double* src, int32_t r, int32_t n, int32_t* changed = nullptr);
 int launch_pack_vec(ppc_state* s, double* dst, const double4* src, int32_t r, int32_t n);
 int launch_unpack_prm(ppc_state* s, int field, const double* src, int32_t r, int32_t n);
+int launch_pull(ppc_state* s);
 int launch_pack_prm(ppc_state* s, int field, double* dst, int32_t first, int32_t n);
 int launch_neighbors_local(ppc_state* s, int32_t r, int32_t n, int32_t* counts, int32_t* lists, int32_t cap);
 int launch_springs_local(ppc_state* s, int32_t r, int32_t n, int32_t* rows, int32_t cap, int to_device);
