@@ -3632,6 +3632,14 @@ __global__ void k_count_flags(view v, int r, int flag, int32_t* count)
 		atomicAdd(count, warp_total);
 }
 
+__global__ void k_bump_spring_epoch(view v)
+{
+	grid_wait();
+	const int r = blockIdx.x * blockDim.x + threadIdx.x;
+	if (r < v.nreps)
+		v.ctr[r].spring_epoch++;
+}
+
 __global__ void k_bump_draw_epoch(view v)
 {
 	grid_wait();
@@ -4278,6 +4286,14 @@ int launch_spring_step(ppc_state* s)
 
 int launch_spring_updates(ppc_state* s)
 {
+	if (!s->rates_nonzero)
+	{
+		// no draw passes a zero rate: only the epoch of the draws advances, as
+		// in the fused steps
+		pdl(k_bump_spring_epoch, blocks_for(s->nreps, kThreads), kThreads, 0, PPC_LAUNCH(s), s->v);
+		PPC_CHECK_LAUNCH();
+		return PPC_OK;
+	}
 	if (int rc = mark_fields_changed(s)) // spring counts change
 		return rc;
 	const int b = blocks_for(s->total_cap, kThreads);
