@@ -560,7 +560,7 @@ def stochastic_springs_form(args, flush):
     out = _timed_steps(sim, stream, sim.step, lambda: a.count, args.steps, args.warmup, flush)
     sim.close()
     out.update({"workload": "config3 + spring rates", "agents": a.count,
-                "note": "attachment 0.8/min, detachment 0.3/min, max 3 springs; separate kernels per step"})
+                "note": "attachment 0.8/min, detachment 0.3/min, max 3 springs; one scan, the settlement and one more pass per step"})
     return out
 
 
