@@ -227,7 +227,7 @@ enum : int
 	LCTL_WANT = 3,	// the same for the next lists: lowered where a pool of entries was too small
 	LCTL_BUILT = 4, // bits of the skin of the lists in use
 	LCTL_FIT = 5,	// every warp has its lists
-	LCTL_LEFT = 6	// steps a launch over lists left to the one behind it
+	LCTL_LEFT = 6	// steps a launch over lists left to k_list_rest behind it
 };
 
 constexpr int32_t kMoved = -2; // view::move_src: the slot's fields changed since the last rebuild
@@ -344,6 +344,7 @@ struct ppc_state
 	int bar_set = 0;			  // barrier words of the next list launch
 	unsigned long long* list_bar = nullptr; // [2 sets * 2 words * 16]
 	bool list_attr[2][2] = {};	  // the list kernels' shared-memory limits are set (per precision and kernel)
+	int rest_blocks[2] = {};	  // blocks of the launch for steps that the lists leave (per precision)
 	std::vector<double> reach_radius, reach_factor; // per replicate: largest uploaded radius and rmad
 	float* pinned_skin = nullptr; // skin of the lists in use, written by the device (0: none)
 	int64_t launches = 0;

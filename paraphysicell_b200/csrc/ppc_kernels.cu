@@ -4547,30 +4547,14 @@ static int list_threads(ppc_state* s)
 	return std::min(kListThreads, std::max(128, (per_sm + 31) / 32 * 32));
 }
 
-template <int DIMS, bool F32, bool RESIDENT, bool LISTED, int MOST>
-static int list_launch_form(ppc_state* s, list_args a, int T)
+static int cooperative_launch(ppc_state* s, void (*k)(view, list_args), int grid, int threads, size_t dyn, list_args a)
 {
 	a.bar = s->list_bar + 32 * s->bar_set;
 	a.bar_next = s->list_bar + 32 * (s->bar_set ^ 1);
 	s->bar_set ^= 1;
-	auto k = k_list_steps<DIMS, F32, RESIDENT, LISTED, MOST>;
-	const size_t warps = T / 32, step = warps * sizeof(list_step_warp);
-	const size_t entry = (size_t)T * (sizeof(double4) + sizeof(int2));
-	a.cached = RESIDENT ? (int)std::min<size_t>(16, (kListSmem - step) / entry) : 0;
-	const size_t dyn = std::max({ sizeof(place_smem), warps * sizeof(list_warp), step + a.cached * entry,
-								  (size_t)kSortCap * sizeof(int32_t) });
-	if (!s->list_attr[F32][LISTED])
-	{
-		int per_sm = 0;
-		PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
-		PPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, T, dyn));
-		if (per_sm < 1)
-			return cuda_fail(cudaErrorInvalidConfiguration, "steps over lists: no block fits an SM");
-		s->list_attr[F32][LISTED] = true;
-	}
 	cudaLaunchConfig_t cfg {};
-	cfg.gridDim = dim3(std::min(s->sm_count, blocks_for(s->total_cap, T)));
-	cfg.blockDim = dim3(T);
+	cfg.gridDim = dim3(grid);
+	cfg.blockDim = dim3(threads);
 	cfg.dynamicSmemBytes = dyn;
 	cfg.stream = PPC_LAUNCH(s);
 	cudaLaunchAttribute at[1];
@@ -4582,15 +4566,55 @@ static int list_launch_form(ppc_state* s, list_args a, int T)
 	return PPC_OK;
 }
 
+template <int DIMS, bool F32, bool RESIDENT, int MOST>
+static int list_launch_form(ppc_state* s, list_args a, int T)
+{
+	auto k = k_list_steps<DIMS, F32, RESIDENT, MOST>;
+	const size_t warps = T / 32, step = warps * sizeof(list_step_warp);
+	const size_t entry = (size_t)T * (sizeof(double4) + sizeof(int2));
+	a.cached = RESIDENT ? (int)std::min<size_t>(16, (kListSmem - step) / entry) : 0;
+	const size_t dyn = std::max({ sizeof(place_smem), warps * sizeof(list_warp), step + a.cached * entry,
+								  (size_t)kSortCap * sizeof(int32_t) });
+	if (!s->list_attr[F32][1])
+	{
+		int per_sm = 0;
+		PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+		PPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, T, dyn));
+		if (per_sm < 1)
+			return cuda_fail(cudaErrorInvalidConfiguration, "steps over lists: no block fits an SM");
+		s->list_attr[F32][1] = true;
+	}
+	return cooperative_launch(s, k, std::min(s->sm_count, blocks_for(s->total_cap, T)), T, dyn, a);
+}
+
+// the launch for the steps that the lists leave; every block must be resident
+template <int DIMS, bool F32>
+static int list_rest_launch(ppc_state* s, const list_args& a)
+{
+	auto k = k_list_rest<DIMS, F32>;
+	const size_t dyn = std::max({ sizeof(queue_smem), sizeof(place_smem), (size_t)kSortCap * sizeof(int32_t) });
+	if (!s->rest_blocks[F32])
+	{
+		int per_sm = 0;
+		PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+		PPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPersistThreads, dyn));
+		if (per_sm < 1)
+			return cuda_fail(cudaErrorInvalidConfiguration, "steps without lists: no block fits an SM");
+		const int want = std::max({ blocks_for(s->total_cap, kPersistThreads), s->nreps, s->v.ntiles });
+		s->rest_blocks[F32] = std::min(per_sm * s->sm_count, want);
+	}
+	return cooperative_launch(s, k, s->rest_blocks[F32], kPersistThreads, dyn, a);
+}
+
 template <int DIMS, bool F32>
 static int list_launch(ppc_state* s, const list_args& a)
 {
 	const int T = list_threads(s);
 	const int rc = (int64_t)T * s->sm_count < s->total_cap
-					   ? list_launch_form<DIMS, F32, false, true, kListLoop>(s, a, kListLoop)
-					   : (T <= kListFew ? list_launch_form<DIMS, F32, true, true, kListFew>(s, a, T)
-										: list_launch_form<DIMS, F32, true, true, kListThreads>(s, a, T));
-	return rc != PPC_OK ? rc : list_launch_form<DIMS, F32, false, false, kListLoop>(s, a, kListLoop);
+					   ? list_launch_form<DIMS, F32, false, kListLoop>(s, a, kListLoop)
+					   : (T <= kListFew ? list_launch_form<DIMS, F32, true, kListFew>(s, a, T)
+										: list_launch_form<DIMS, F32, true, kListThreads>(s, a, T));
+	return rc != PPC_OK ? rc : list_rest_launch<DIMS, F32>(s, a);
 }
 
 int launch_list_steps(ppc_state* s, int steps)

@@ -187,8 +187,8 @@ __device__ __forceinline__ void list_entry(const view& v, int64_t e, int t, int 
 // and shared out over the lanes (as in the queue pass), so the filter runs on
 // full warps; it runs twice, first to count the entries, then to store them
 // in candidate order, which is that of the mesh. A warp's lists take one slab
-// of the pool, entry k of lane l at k * 32 + l; a warp that finds the pool
-// full scans the mesh instead (and the next lists get a smaller skin). The
+// of the pool, entry k of lane l at k * 32 + l; where a warp finds the pool
+// full, the lists are made again with a smaller skin. The
 // single-precision filter with the replicate's margin never drops a pair
 // within reach plus skin. Every lane calls it.
 // ROUNDS: candidate rounds whose loads are in flight together.
@@ -339,8 +339,6 @@ __device__ __forceinline__ void list_build(const view& v, int cur, int p, int tw
 		w.cnt[lane] = 0;
 		__syncwarp();
 	}
-	if (slab < 0 && act)
-		v.nlc[t] = c; // its stencil's agents
 	if (lane == 0 && tw < n)
 	{
 		v.nl_slab[tw >> 5] = slab;
@@ -609,60 +607,17 @@ struct list_cache
 	int T, t0; // threads of the block, and the key-ordered position of its first
 };
 
-// Candidate k of the agent at t, whose warp has no lists: the agents of its
-// stencil's voxels in the mesh the lists were to be made from, itself among
-// them. Rare, so it is found anew each time and keeps no registers.
-template <int DIMS>
-__device__ __forceinline__ int2 list_candidate(const view& v, int t, int k)
-{
-	const int r = rep_of(v, max(v.sorted[t], 0));
-	const rep_info& R = v.reps[r];
-	int cx, cy, cz;
-	voxel_coords(R, (int32_t)(v.skey[t] - R.vox_base), cx, cy, cz);
-	const int xlo = max(cx - 1, 0), xhi = min(cx + 1, R.grid[0] - 1);
-#pragma unroll 1
-	for (int row = 0; row < (DIMS == 3 ? 9 : (DIMS == 2 ? 3 : 1)); row++)
-	{
-		const int z = cz + (DIMS == 3 ? row / 3 - 1 : 0), y = cy + (DIMS >= 2 ? row % 3 - 1 : 0);
-		if (z < 0 || z >= R.grid[2] || y < 0 || y >= R.grid[1])
-			continue;
-		const int32_t key = (int32_t)R.vox_base + R.grid[0] * (y + R.grid[1] * z);
-		const int lo = v.vstart[key + xlo], n = v.vstart[key + xhi + 1] - lo;
-		if (k < n)
-		{
-			const int u = lo + k;
-			const bool mov = ((__double_as_longlong(v.sprm4[u].w) >> 32) & 1) != 0;
-			return make_int2(u | (mov ? 0 : kStill), __float_as_int((float)(v.spos4[t].w + v.spos4[u].w)));
-		}
-		k -= n;
-	}
-	return make_int2(t, 0);
-}
-
-// entry k of the agent at t, in its warp's slab (LISTED: it has one); where
-// entries are cached, the agent's thread is t less the block's first
-template <int DIMS, bool LISTED>
+// entry k of the agent at t, in its warp's slab; where entries are cached, the
+// agent's thread is t less the block's first
 __device__ __forceinline__ int2 list_get(const view& v, const list_cache& lc, int64_t slab, int t, int k)
 {
-	if (!LISTED)
-		return list_candidate<DIMS>(v, t, k);
 	return k < lc.n ? lc.entry[k * lc.T + t - lc.t0] : v.nl[slab + (t & 31) + 32 * k];
 }
 
-// what the pair code needs of the agent at t and its entry k, neighbour u
-template <bool F32, bool LISTED>
-__device__ __forceinline__ double4 list_get_pair(const view& v, const list_cache& lc, int64_t slab, int t, int k,
-												 int u)
+// what the pair code needs of the agent at t and its entry k
+template <bool F32>
+__device__ __forceinline__ double4 list_get_pair(const view& v, const list_cache& lc, int64_t slab, int t, int k)
 {
-	if (!LISTED)
-	{
-		const double4 qi = v.sprm4[t], qj = v.sprm4[u];
-		int def_i, def_j;
-		bool mov_i, mov_j;
-		unpack_bits(qi.w, def_i, mov_i);
-		unpack_bits(qj.w, def_j, mov_j);
-		return list_pair<F32>(v, t, u, qi, qj, v.spos4[t].w, v.spos4[u].w, def_i, def_j);
-	}
 	const int64_t e = slab + (t & 31) + 32 * k;
 	if (F32)
 	{
@@ -762,7 +717,7 @@ __device__ __forceinline__ void list_enter(const view& v, const list_args& a, co
 // on after the last one in the order. `first`: flags and entry velocities
 // count; `last`: the slot-ordered rows are stored. Returns the step's events.
 // Every lane calls it.
-template <int DIMS, bool F32, int BATCH, bool LISTED>
+template <int DIMS, bool F32, int BATCH>
 __device__ __forceinline__ unsigned long long list_step(const view& v, const list_args& a, const rep_info* reps,
 														const list_cache& lc, list_step_warp& w, const list_own& o,
 														int p, int t, int n, bool first, bool last, float skin)
@@ -802,7 +757,7 @@ __device__ __forceinline__ unsigned long long list_step(const view& v, const lis
 #pragma unroll
 				for (int j = 0; j < BATCH; j++)
 					if (k0 + BATCH + j < cnt)
-						next[j] = list_get<DIMS, LISTED>(v, lc, o.slab, t, k0 + BATCH + j);
+						next[j] = list_get(v, lc, o.slab, t, k0 + BATCH + j);
 				if (k0 < 0)
 					continue;
 #pragma unroll
@@ -812,7 +767,7 @@ __device__ __forceinline__ unsigned long long list_step(const view& v, const lis
 						continue;
 					const int u = e[j].x & ~kStill;
 					const int in = list_test<DIMS>(pi, q[j], __int_as_float(e[j].y));
-					if (in == 0 || (!LISTED && u == t) || (in < 0 && !list_near<DIMS>(pi, q[j], v.spos4[t].w + v.spos4[u].w)))
+					if (in == 0 || (in < 0 && !list_near<DIMS>(pi, q[j], v.spos4[t].w + v.spos4[u].w)))
 						continue;
 					const unsigned long long ow = (unsigned long long)__double_as_longlong(q[j].w);
 					if (ow <= done)
@@ -820,7 +775,7 @@ __device__ __forceinline__ unsigned long long list_step(const view& v, const lis
 					more = more || nh == kListHits;
 					if (nh == kListHits && ow > tail)
 						continue;
-					if (LISTED && k0 + j >= lc.n)
+					if (k0 + j >= lc.n)
 						prefetch_l1(v.nl_pair + o.slab + lane + 32 * (k0 + j));
 					// at the end of the hits, or, where agents crossed voxels
 					// since the lists were made, at its place among them
@@ -862,7 +817,7 @@ __device__ __forceinline__ unsigned long long list_step(const view& v, const lis
 						i += step;
 				const int2 hit = w.hit[x - w.first[i]][i];
 				const int u = hit.y;
-				const double4 pair = list_get_pair<F32, LISTED>(v, lc, o.slab, t - lane + i, hit.x, u & ~kStill); // one slab per warp
+				const double4 pair = list_get_pair<F32>(v, lc, o.slab, t - lane + i, hit.x); // one slab per warp
 				mov_j = (u & kStill) == 0;
 				const double4 tm = list_terms<DIMS, F32>(make_double4(w.px[i], w.py[i], w.pz[i], 0.0),
 														 row_load(pos + (u & ~kStill)),
@@ -1202,28 +1157,22 @@ __device__ __forceinline__ bool list_rebuild(const view& v, const list_args& a, 
 
 // The steps of a call. RESIDENT: the grid has a thread for every agent, which
 // keeps the agent's rows and the first entries of its list in shared memory
-// between the steps. LISTED: the launch runs while every warp has its lists;
-// where some do not fit, the rest of the call is left (LCTL_LEFT) to the
-// launch behind it, whose agents scan the mesh. (One kernel with both bodies
-// spilled registers in the listed one: 29,000 cycles a step on 88,700 agents
-// instead of 22,000. The second launch costs a call about 3 us.)
-template <int DIMS, bool F32, bool RESIDENT, bool LISTED, int MOST>
+// between the steps. The launch runs while every warp has its lists; where
+// some do not fit, or no skin is left, it leaves the rest of the call
+// (LCTL_LEFT), with the mesh current, to k_list_rest behind it.
+template <int DIMS, bool F32, bool RESIDENT, int MOST>
 __global__ void __launch_bounds__(MOST, 1)
 	k_list_steps(const __grid_constant__ view v, const __grid_constant__ list_args a)
 {
 	// list entries whose loads are in flight together: as many as the
 	// registers of MOST threads hold
-	constexpr int BATCH = !LISTED ? 1 : MOST > kListFew ? 2 : 4;
+	constexpr int BATCH = MOST > kListFew ? 2 : 4;
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ rep_info s_rep;
 	if (ld_relaxed_i32(v.err) & ERR_TIMEOUT)
 		return; // an earlier launch gave up: wait for the host
 	if (blockIdx.x == 0 && threadIdx.x < 2)
 		a.bar_next[16 * threadIdx.x] = 0;
-	const int steps = LISTED ? a.steps : v.lctl[LCTL_LEFT];
-	if (!LISTED && steps == 0)
-		return;
-	const int k0 = a.steps - steps; // steps of the call done before this launch
 	const int T = blockDim.x, t0 = blockIdx.x * T + threadIdx.x, step = gridDim.x * T;
 	if (v.nreps == 1 && threadIdx.x == 0)
 		s_rep = v.reps[0];
@@ -1240,10 +1189,10 @@ __global__ void __launch_bounds__(MOST, 1)
 		bar = list_barrier {};
 	__syncthreads();
 	int n = *v.cursor;
-	int p = a.p ^ (k0 & 1);
+	int p = a.p;
 	float skin = lctl_float(v, LCTL_BUILT);
 	bool rebuild = v.lctl[LCTL_DIRTY] != 0 || lctl_float(v, LCTL_WANT) < skin;
-	if (LISTED && a.refresh)
+	if (a.refresh)
 	{
 		unsigned long long ev = 0;
 		for (int t = t0; t < n; t += step)
@@ -1272,8 +1221,8 @@ __global__ void __launch_bounds__(MOST, 1)
 		}
 		__syncwarp();
 	};
-	bool flushed = k0 == 0, replay = false; // of the rebuild: the slot-ordered rows are current; removals are due
-	for (int k = k0;; k++)
+	bool flushed = true, replay = false; // of the rebuild: the slot-ordered rows are current; removals are due
+	for (int k = 0;; k++)
 	{
 		if (rebuild)
 		{
@@ -1282,7 +1231,7 @@ __global__ void __launch_bounds__(MOST, 1)
 			n = *v.cursor;
 			skin = lctl_float(v, LCTL_BUILT);
 		}
-		if (LISTED && (k == 0 || rebuild))
+		if (k == 0 || rebuild)
 		{
 			const bool fit = v.lctl[LCTL_FIT] != 0;
 			if (t0 == 0)
@@ -1297,14 +1246,14 @@ __global__ void __launch_bounds__(MOST, 1)
 		const bool last = k == a.steps - 1;
 		unsigned long long ev = 0;
 		if (RESIDENT)
-			ev = list_step<DIMS, F32, BATCH, LISTED>(v, a, reps, lc, w, own, p, t0, n, k == 0, last, skin);
+			ev = list_step<DIMS, F32, BATCH>(v, a, reps, lc, w, own, p, t0, n, k == 0, last, skin);
 		else
 			for (int tb = blockIdx.x * T; tb < n; tb += step)
 			{
 				const int t = tb + threadIdx.x;
 				own = list_load(v, a, w, p, t, n);
 				list_prefetch(v, p, (t & ~31) + step, n);
-				ev |= list_step<DIMS, F32, BATCH, LISTED>(v, a, reps, lc, w, own, p, t, n, k == 0, last, skin);
+				ev |= list_step<DIMS, F32, BATCH>(v, a, reps, lc, w, own, p, t, n, k == 0, last, skin);
 			}
 		p ^= 1;
 		ev = list_wait(v, a, bar, ev);
@@ -1331,5 +1280,73 @@ __global__ void __launch_bounds__(MOST, 1)
 	}
 	if (blockIdx.x == 0 && v.auto_springs)
 		for (int r = threadIdx.x; r < v.nreps; r += T)
-			v.ctr[r].spring_epoch += a.steps; // (the launch that ends the call counts all of them)
+			v.ctr[r].spring_epoch += a.steps;
+}
+
+// The steps that k_list_steps left, without lists: the queue pass over the
+// mesh, the container update and the mesh rebuild, separated by grid barriers,
+// as in the persistent step (whose registers and blocks per SM bound it the
+// same way). Its own kernel, since one with both bodies spilled registers in
+// the steps over lists (29,000 cycles a step on 88,700 agents instead of
+// 22,000); where nothing is left the launch costs a call about 3 us. The slot-
+// ordered positions end in pos[a.cur], and the next lists start from a
+// rebuild.
+template <int DIMS, bool F32>
+__global__ void __launch_bounds__(kPersistThreads)
+	k_list_rest(const __grid_constant__ view v, const __grid_constant__ list_args a)
+{
+	extern __shared__ __align__(16) unsigned char smem[];
+	if (ld_relaxed_i32(v.err) & ERR_TIMEOUT)
+		return; // an earlier launch gave up: wait for the host
+	if (blockIdx.x == 0 && threadIdx.x < 2)
+		a.bar_next[16 * threadIdx.x] = 0;
+	const int steps = v.lctl[LCTL_LEFT];
+	if (steps == 0)
+		return;
+	__shared__ list_barrier bar;
+	if (threadIdx.x == 0)
+		bar = list_barrier {};
+	__syncthreads();
+	const int T = kPersistThreads, t0 = blockIdx.x * T, step = gridDim.x * T;
+	int cur = a.cur;
+	for (int k = a.steps - steps; k < a.steps; k++)
+	{
+		const int opts = k == 0 ? a.opts : a.opts & ~FUSED_VEL, nxt = cur ^ 1;
+		for (int t = t0; t < v.total_cap; t += step)
+			fused_queue_agent<DIMS, F32>(v, cur, opts, t + threadIdx.x,
+										 reinterpret_cast<queue_smem*>(smem)->w[threadIdx.x >> 5]);
+		if (list_wait(v, a, bar, 0) == ~0ull)
+			return;
+		for (int r = blockIdx.x; r < v.nreps; r += gridDim.x)
+		{
+			compact_plan_rep(v, r, 0, a.springs, 1, 0, reinterpret_cast<int32_t*>(smem));
+			__syncthreads(); // thread 0 finishes the serial plan before the next sort
+		}
+		if (blockIdx.x == 0 && threadIdx.x == 0)
+			*v.bin_active = 1;
+		if (list_wait(v, a, bar, 0) == ~0ull)
+			return;
+		for (int t = t0; t < v.total_cap; t += step)
+			bin_count_body(v, nxt, t + threadIdx.x);
+		if (list_wait(v, a, bar, 0) == ~0ull)
+			return;
+		for (int b = blockIdx.x; b < v.ntiles; b += gridDim.x)
+			bin_order_tile<kPersistThreads>(v, b, *reinterpret_cast<place_smem*>(smem), 1);
+		if (list_wait(v, a, bar, 0) == ~0ull)
+			return;
+		for (int t = t0; t < v.total_cap; t += step)
+			bin_copy_agent(v, nxt, t + threadIdx.x, 0, v.spos4, v.sposf, 1);
+		bin_finish(v, t0 + threadIdx.x, step);
+		if (list_wait(v, a, bar, 0) == ~0ull)
+			return;
+		cur = nxt;
+	}
+	if (cur != a.cur)
+		for (int t = t0 + threadIdx.x; t < v.total_cap; t += step)
+			v.pos[a.cur][t] = v.pos[cur][t];
+	if (blockIdx.x == 0 && threadIdx.x == 0)
+		v.lctl[LCTL_DIRTY] = 1;
+	if (blockIdx.x == 0 && v.auto_springs)
+		for (int r = threadIdx.x; r < v.nreps; r += T)
+			v.ctr[r].spring_epoch += a.steps;
 }

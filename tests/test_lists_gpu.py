@@ -133,6 +133,31 @@ def test_reach_that_leaves_no_skin(form):
     d.close()
 
 
+@pytest.mark.parametrize("form", FORMS)
+@pytest.mark.parametrize("steps", [7, 12])
+def test_reach_that_leaves_no_skin_and_goes_with_its_agents(form, steps):
+    """The agents whose ingestions took the skin are removed in the first step
+    of a call: the mesh rebuilt after it would leave a skin again, and the rest
+    of the call sees every neighbour all the same (odd and even numbers of
+    steps are left to the pass without lists)."""
+    mesh, params, a = _agents(800, 3, 110, 31, FORMS[form], radius=(9.5, 11.0))
+    f = wl.interaction_fields(a, 2, 4, scale=40.0)
+    o, d = make_pair(mesh, params, a)
+    _mesh(o, d)
+    for x in (o, d):
+        x.update_cell_cell_interactions(f.copy())
+        x.update_cell_container_for_mechanics()
+    h = fetch(d, a)
+    grown = 2 * 1.25 * h["radius"] > 29.0
+    assert 0 < grown.sum() < h.count // 2
+    h["flags"][grown] = 1
+    o.upload(h)
+    d.upload_fields(h, ("flags",))
+    _run(o, d, a, (steps, 5))
+    assert fetch(d, a).count <= h.count - grown.sum()
+    d.close()
+
+
 def test_fp32_force_lists_match_the_scanning_pass():
     """The FP32-force form over lists adds the same terms in the same order as
     its scanning passes, so the two agree bit for bit."""
