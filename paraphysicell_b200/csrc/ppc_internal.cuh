@@ -343,7 +343,7 @@ struct ppc_state
 	int lcur = 0;				  // lpos buffer that holds the positions
 	int bar_set = 0;			  // barrier words of the next list launch
 	unsigned long long* list_bar = nullptr; // [2 sets * 2 words * 16]
-	bool list_attr[2][2] = {};	  // the list kernels' shared-memory limits are set (per precision and kernel)
+	bool list_ready[2] = {};	  // the list kernel's shared-memory limit is set (per precision)
 	int rest_blocks[2] = {};	  // blocks of the launch for steps that the lists leave (per precision)
 	std::vector<double> reach_radius, reach_factor; // per replicate: largest uploaded radius and rmad
 	float* pinned_skin = nullptr; // skin of the lists in use, written by the device (0: none)

@@ -4575,14 +4575,19 @@ static int list_launch_form(ppc_state* s, list_args a, int T)
 	a.cached = RESIDENT ? (int)std::min<size_t>(16, (kListSmem - step) / entry) : 0;
 	const size_t dyn = std::max({ sizeof(place_smem), warps * sizeof(list_warp), step + a.cached * entry,
 								  (size_t)kSortCap * sizeof(int32_t) });
-	if (!s->list_attr[F32][1])
+	static_assert(sizeof(place_smem) <= kListSmem && MOST / 32 * sizeof(list_warp) <= kListSmem
+					  && kSortCap * sizeof(int32_t) <= kListSmem,
+				  "the limit below holds for every block size");
+	if (!s->list_ready[F32])
 	{
+		// The limit belongs to the kernel, which all states share, whereas
+		// `dyn` follows the state's capacity: every state sets the same one.
 		int per_sm = 0;
-		PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn));
+		PPC_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kListSmem));
 		PPC_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, T, dyn));
 		if (per_sm < 1)
 			return cuda_fail(cudaErrorInvalidConfiguration, "steps over lists: no block fits an SM");
-		s->list_attr[F32][1] = true;
+		s->list_ready[F32] = true;
 	}
 	return cooperative_launch(s, k, std::min(s->sm_count, blocks_for(s->total_cap, T)), T, dyn, a);
 }

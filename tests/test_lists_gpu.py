@@ -158,6 +158,24 @@ def test_reach_that_leaves_no_skin_and_goes_with_its_agents(form, steps):
     d.close()
 
 
+@pytest.mark.parametrize("capacities", [(1000, 30000), (30000, 1000), (42000, 90000), (90000, 42000)])
+def test_two_live_states_of_different_capacity(capacities):
+    """Both states run the same kernel with shared memory by their own
+    capacity, in turn."""
+    pairs = []
+    for k, c in enumerate(capacities):
+        mesh, params, a = _agents(600, 3, 110, 41 + k, c)
+        pairs.append((*make_pair(mesh, params, a), a))
+        _mesh(pairs[-1][0])
+    for _ in range(3):
+        for o, d, a in pairs:
+            o.step(5, 0, 0.0, 0.0)
+            d.step(5)
+            assert_same_state(fetch(d, a), fetch(o, a))
+    for o, d, a in pairs:
+        d.close()
+
+
 def test_fp32_force_lists_match_the_scanning_pass():
     """The FP32-force form over lists adds the same terms in the same order as
     its scanning passes, so the two agree bit for bit."""
