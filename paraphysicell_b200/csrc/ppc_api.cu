@@ -381,6 +381,13 @@ const void* mapped(const void* host)
 	return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
 }
 
+// the same for rows of doubles: null where a kernel's loads of them would be
+// misaligned (a copy takes any address)
+const void* mapped_doubles(const void* host)
+{
+	return reinterpret_cast<uintptr_t>(host) % sizeof(double) == 0 ? mapped(host) : nullptr;
+}
+
 // Host rows (dims doubles per agent) into the double4 device rows. Pinned
 // host buffers go through the copy engine into the staging arena (or, in the
 // zero-copy transfer mode, are read by the unpack kernel over the bus);
@@ -393,7 +400,7 @@ int put_vec(ppc_state* s, double4* dev, const double* host, int32_t r, int32_t n
 	if (n == 0)
 		return PPC_OK;
 	if (host && (s->zero_copy || s->direct_rows))
-		if (const void* d = mapped(host))
+		if (const void* d = mapped_doubles(host))
 			return launch_unpack_vec(s, dev, static_cast<const double*>(d), r, n, changed);
 	const size_t bytes = (size_t)n * s->dims * sizeof(double);
 	void* st = nullptr;
@@ -418,7 +425,7 @@ int get_vec(ppc_state* s, double* host, const double4* dev, int32_t r, int32_t f
 	if (pull_column(s, host, dev + s->reps[r].base, (size_t)n * s->dims * sizeof(double), s->dims))
 		return PPC_OK;
 	if (s->zero_copy)
-		if (const void* d = mapped(host))
+		if (const void* d = mapped_doubles(host))
 			return launch_pack_vec(s, static_cast<double*>(const_cast<void*>(d)), dev, r, n);
 	const size_t bytes = (size_t)n * s->dims * sizeof(double);
 	void* st = nullptr;

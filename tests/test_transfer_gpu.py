@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from paraphysicell_b200 import workloads as wl
-from paraphysicell_b200.abi import AgentArrays
+from paraphysicell_b200.abi import PPC_TRANSFER_COPY_ENGINE, PPC_TRANSFER_ZERO_COPY, AgentArrays
 from paraphysicell_b200.device import PinnedPool, Simulation
 from tests import gpu_util as gu
 
@@ -111,3 +111,38 @@ def test_download_after_other_work_waits_for_it():
     gu.assert_same_state(got, gu.fetch(o, a))
     assert np.count_nonzero(got["flags"][: got.count]) > 0
     d.close()
+
+
+@pytest.mark.parametrize("mode", [PPC_TRANSFER_COPY_ENGINE, PPC_TRANSFER_ZERO_COPY])
+@pytest.mark.parametrize("n", [33, 3000])
+def test_page_locked_rows_off_the_alignment_of_doubles(n, mode):
+    """Rows that start four bytes past a double's boundary take the copies,
+    both ways, at the size the kernels would otherwise read and at a larger
+    one."""
+    mesh, params, a = wl.scaled(wl.config2, n, seed=19)
+    o, d = gu.make_pair(mesh, params, a)
+    d.set_host_transfer(mode)
+    pool = PinnedPool()
+    h = gu.fetch(d, a)
+    fields = ("positions", "previous_velocities", "simple_pressure")
+    for f in fields:
+        raw = pool(8 * h.arrays[f].size + 4, np.uint8)
+        rows = raw[4:].view(np.float64)
+        assert rows.ctypes.data % 8 == 4
+        rows[:] = h.arrays[f]
+        h.arrays[f] = rows
+    h.arrays["positions"][:] *= 0.99
+    o.upload(h)
+    o.update_mechanics_mesh()
+    o.update_cell_neighbors()
+    d.upload_fields(h, fields[:2])
+    for _ in range(2):
+        d.step(1)
+        o.step(1, 0, 0.0, 0.0)
+        d.download(h, fields=fields)
+        gu.assert_same_state(gu.fetch(d, a), gu.fetch(o, a))
+        for f in fields:
+            assert np.array_equal(h[f], gu.fetch(d, a)[f])
+        d.upload_fields(h, fields[:2])
+    d.close()
+    pool.free()
