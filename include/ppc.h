@@ -581,12 +581,15 @@ int ppc_get_profile(ppc_state* s, double* fused_ms, int64_t* fused_launches);
  * PPC_NOALLOC_MAX_VOXELS return PPC_ERR_CAPACITY (the grid is sized in 64-bit
  * arithmetic, so no mesh extent can wrap it). The in-voxel ordering pass costs
  * c^2 loads for a voxel of c agents: negligible at tissue densities, about a
- * second of GPU time if all PPC_NOALLOC_MAX_AGENTS agents share one voxel.
- * Nothing is allocated. The
- * first call on a device looks the array's address up for that device, so
- * make that first call before any stream capture. All calls share the array:
- * calls whose work overlaps on the GPU race. Work is queued on `cuda_stream`
- * (NULL: the legacy default stream) and the call returns without waiting. */
+ * second of GPU time if all PPC_NOALLOC_MAX_AGENTS agents share one voxel. Nothing is allocated. The first call on a device
+ * looks the array's address up for that device, so make that first call
+ * before any stream capture. All calls on a device share the array: calls on
+ * different streams run one after another (an event orders them), but graph
+ * replays of captured calls must not overlap with other calls or replays,
+ * whose outputs they would spoil. Work is queued on `cuda_stream` (NULL: the
+ * legacy default stream) and the call returns without waiting. Its device
+ * waits are bounded; if one gave up (on a GPU that makes no progress for
+ * seconds), voxel_counts[0] is -1 and the results are incomplete. */
 int ppc_bin_agents_noalloc(const ppc_mesh* mesh, const double* positions, int32_t count, int32_t* voxel_counts,
 						   int32_t* agents, void* cuda_stream);
 

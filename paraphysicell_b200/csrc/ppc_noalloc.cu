@@ -9,10 +9,14 @@
 // intermediate (per-voxel chains and prefix, totals of voxel ranges) in
 // g_noalloc_scratch below, a fixed-size array in device memory.
 // Every GPU that loads this library reserves that array until the process
-// exits. All calls share it and it keeps the previous call's contents; every
-// entry is rewritten before it is read, so nothing has to be cleared between
-// calls, but calls whose work overlaps on the GPU (different streams, or
-// different host threads on one device) race on it.
+// exits. All calls on a device share it and it keeps the previous call's
+// contents; every entry is rewritten before it is read, apart from the words
+// that order a call's work (na_words), which the call before it clears. Calls
+// on different streams are ordered one after another by an event. Calls
+// captured into graphs are not: replays that overlap with each other or with
+// other calls race on the scratch and spoil each other's outputs, though
+// nothing beyond those (their words are cleared before every replay, and no
+// index read from the scratch is used unchecked).
 //
 // The result is the one ppc_update_mechanics_mesh + ppc_get_mesh_bins give:
 // per-voxel counts and the agents grouped by voxel in voxel order, in
@@ -28,20 +32,22 @@
 namespace {
 
 constexpr int kNaThreads = 1024;
-constexpr int64_t kNaBlocks = 1024; // more than any grid has
+constexpr int kNaBlocks = 1024; // more than any grid has
 constexpr int kNaChain = 24; // agents of a voxel whose order their chain gives; larger voxels are sorted by a block
 constexpr int kNaSort = 4096; // agents of one voxel sorted in shared memory
-constexpr long long kNaWait = 1LL << 25; // polls of a barrier before it gives up
+constexpr int kNaWait = 1 << 22; // polls of a wait before it gives up, about two seconds
 
 // layout of the scratch, in int32 units
 constexpr int64_t kOffNext = 0;
-constexpr int64_t kOffBig = kOffNext + PPC_NOALLOC_MAX_AGENTS; // voxels whose agents a block sorts
+constexpr int64_t kOffKey = kOffNext + PPC_NOALLOC_MAX_AGENTS;
+constexpr int64_t kOffBig = kOffKey + PPC_NOALLOC_MAX_AGENTS; // voxels whose agents a block sorts
 constexpr int64_t kOffHead = kOffBig + PPC_NOALLOC_MAX_AGENTS;
 constexpr int64_t kOffStart = kOffHead + PPC_NOALLOC_MAX_VOXELS;
 constexpr int64_t kOffTile = kOffStart + PPC_NOALLOC_MAX_VOXELS;
 constexpr int64_t kOffNbig = kOffTile + kNaBlocks;
-constexpr int64_t kOffBarrier = kOffNbig + 32; // arrivals, and 32 words on the generation
-constexpr int64_t kScratchInts = kOffBarrier + 64;
+constexpr int64_t kOffWords = kOffNbig + 32; // na_words: two that calls use in turn, and the captured calls'
+constexpr int64_t kWordsInts = 2 * 32;
+constexpr int64_t kScratchInts = kOffWords + 3 * kWordsInts;
 
 static __device__ __align__(256) int32_t g_noalloc_scratch[kScratchInts];
 
@@ -63,38 +69,34 @@ __device__ __forceinline__ int na_axis(double x, const na_mesh& m, int d)
 	return (int)q;
 }
 
-// Grid barrier: the last block to arrive clears the arrivals and moves the
-// generation on, which the others poll, so the words need no reset between
-// launches. False when the wait gave up (the grid is resident: it does not).
-__device__ bool na_barrier(int32_t* scratch)
+// The words that order one call's work, a line each: items handed out and
+// items done.
+struct na_words
 {
-	__shared__ int s_ok;
-	__syncthreads();
-	if (threadIdx.x == 0)
+	int32_t ticket, pad0[31], done, pad1[31];
+};
+static_assert(sizeof(na_words) == kWordsInts * sizeof(int32_t), "one line per word");
+
+// Thread 0 waits until `want` items are done; false when it gave up. The item
+// it then leaves undone makes every block that needs it give up as well, and
+// each of them marks the counts with a value that no voxel has as its last
+// act, so the mark stands when the launch ends.
+__device__ __forceinline__ bool na_wait(na_words* w, int want, int32_t* counts)
+{
+	int x, polls = 0;
+	while (true)
 	{
-		unsigned* arrivals = reinterpret_cast<unsigned*>(scratch + kOffBarrier);
-		unsigned* gen = arrivals + 32;
-		unsigned g, at, x;
-		asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(g) : "l"(gen) : "memory");
-		asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;" : "=r"(at) : "l"(arrivals) : "memory");
-		s_ok = 1;
-		if (at == gridDim.x - 1)
+		asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(x) : "l"(&w->done) : "memory");
+		if (x >= want)
+			break;
+		if (++polls >= kNaWait)
 		{
-			asm volatile("st.relaxed.gpu.global.u32 [%0], 0;" ::"l"(arrivals) : "memory");
-			asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(gen) : "memory");
+			atomicExch(counts, -1);
+			return false;
 		}
-		else
-		{
-			long long polls = 0;
-			do
-				asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(x) : "l"(gen) : "memory");
-			while (x == g && ++polls < kNaWait);
-			s_ok = x != g;
-		}
-		asm volatile("fence.acq_rel.gpu;" ::: "memory");
 	}
-	__syncthreads();
-	return s_ok != 0;
+	asm volatile("fence.acq_rel.gpu;" ::: "memory");
+	return true;
 }
 
 __device__ __forceinline__ int na_block_scan(int x, int& total)
@@ -178,144 +180,184 @@ __device__ void na_sort(int32_t* agents, int c, int32_t* copy, int32_t* sh)
 	__syncthreads();
 }
 
-// The whole call as one cooperative launch with a thread per agent and three
-// grid barriers: clear, count, scan, place. The call moves 6 MB for 100,003
-// agents in 884,736 voxels and is bound by its dependent phases: a memset and
-// five launches took 35.8 us (31.5 us of it on the host), five launches whose
-// waits overlapped the same, this kernel with an atomic per agent on its
-// range's total 36.9 us, and with the totals summed per block first 20.5 us,
-// of whose 33,000 cycles the barriers take 15,000.
+// The whole call as one launch. The phases clear, count, scan, place and
+// sort have an item per block each. A block takes the items in their order
+// off a counter, whatever its index, and an item starts once every item of the
+// phases before is done. So an item waits only for items that blocks already
+// running have taken: the launch needs no set of blocks resident at once, and
+// runs beside a kernel that holds some of the SMs. It clears `after`, the words
+// of the call behind it.
+//
+// The call moves 6 MB for 100,003 agents in 884,736 voxels and is bound by its
+// dependent phases: a memset and five launches take 34.2 us, one
+// launch with grid barriers (which needs all its blocks resident) 20.5, this one
+// 20.6 to 21.2 us.
 //  count: an agent's voxel, and its link on the voxel's chain. The chain's
 //   last link is whatever the scratch held: whoever walks it knows the count.
 //   The totals of the blocks' voxel ranges are formed here too.
-//  scan: each block the starts of its range of voxels.
+//  scan: the starts of a range of voxels.
 //  place: descending index inside the voxel, from the agents on its chain; an
 //   agent of a voxel of more than kNaChain takes its place on the chain, and a
-//   block sorts the voxel.
+//   block sorts the voxel in the last phase.
 __global__ void __launch_bounds__(kNaThreads, 1)
-	k_na_bins(const double* __restrict__ pos, int n, na_mesh m, int32_t* counts, int32_t* scratch, int32_t* agents)
+	k_na_bins(const double* __restrict__ pos, int n, na_mesh m, int32_t* counts, int32_t* scratch, na_words* words,
+			  na_words* after, int32_t* agents)
 {
 	__shared__ int32_t sh[kNaSort];
-	const int t = blockIdx.x * kNaThreads + threadIdx.x, stride = gridDim.x * kNaThreads;
+	__shared__ int s_next, s_ok, s_all;
+	const int G = gridDim.x, stride = G * kNaThreads;
 	const int nvox = m.nvox;
-	// voxels per block, a multiple of four
-	const int range = ((nvox + gridDim.x - 1) / gridDim.x + 3) & ~3;
-
-	// the caller's buffer is 4-byte aligned at least
-	const int head = min(nvox, (int)((16 - (reinterpret_cast<uintptr_t>(counts) & 15)) & 15) / 4);
-	const int n4 = (nvox - head) / 4;
-	for (int k = t; k < n4; k += stride)
-		reinterpret_cast<int4*>(counts + head)[k] = make_int4(0, 0, 0, 0);
-	if (t < head)
-		counts[t] = 0;
-	if (t < nvox - head - 4 * n4)
-		counts[head + 4 * n4 + t] = 0;
-	if (t < gridDim.x)
-		scratch[kOffTile + t] = 0;
-	if (t == 0)
-		scratch[kOffNbig] = 0;
-	if (!na_barrier(scratch))
-		return;
-
-	// the grid holds PPC_NOALLOC_MAX_AGENTS threads on a whole GPU; smaller
-	// ones take agents in turn and look their voxel up again
-	auto voxel = [&](int i) {
-		const int c0 = na_axis(pos[(int64_t)i * m.dims], m, 0);
-		const int c1 = m.dims >= 2 ? na_axis(pos[(int64_t)i * m.dims + 1], m, 1) : 0;
-		const int c2 = m.dims >= 3 ? na_axis(pos[(int64_t)i * m.dims + 2], m, 2) : 0;
-		return c0 + m.grid[0] * (c1 + m.grid[1] * c2);
-	};
-	int key = 0;
-	for (int k = threadIdx.x; k < gridDim.x; k += kNaThreads)
-		sh[k] = 0;
-	__syncthreads();
-	for (int i = t; i < n; i += stride)
+	// voxels per item of the scan, a multiple of four
+	const int range = ((nvox + G - 1) / G + 3) & ~3;
+	int next = 0;
+	if (threadIdx.x == 0)
+		next = atomicAdd(&words->ticket, 1);
+	while (true)
 	{
-		key = voxel(i);
-		atomicAdd(counts + key, 1);
-		const int before = atomicExch(scratch + kOffHead + key, i);
-		atomicAdd(sh + key / range, 1);
-		scratch[kOffNext + i] = before;
-	}
-	__syncthreads();
-	for (int k = threadIdx.x; k < gridDim.x; k += kNaThreads)
-		if (sh[k])
-			atomicAdd(scratch + kOffTile + k, sh[k]);
-	if (!na_barrier(scratch))
-		return;
-
-	int part = 0;
-	for (int k = threadIdx.x; k < blockIdx.x; k += kNaThreads)
-		part += scratch[kOffTile + k];
-	const int lo = blockIdx.x * range, hi = min(nvox, lo + range);
-	int c[4];
-	auto load = [&](int i) {
-#pragma unroll
-		for (int q = 0; q < 4; q++)
-			c[q] = i + q < hi ? counts[i + q] : 0;
-	};
-	load(lo + 4 * threadIdx.x);
-	int base;
-	na_block_scan(part, base);
-	for (int b = lo; b < hi; b += 4 * kNaThreads)
-	{
-		const int i = b + 4 * threadIdx.x;
-		if (b > lo)
-			load(i);
-		int total;
-		int4 out;
-		out.x = base + na_block_scan(c[0] + c[1] + c[2] + c[3], total);
-		out.y = out.x + c[0];
-		out.z = out.y + c[1];
-		out.w = out.z + c[2];
-		if (i + 3 < hi)
-			*reinterpret_cast<int4*>(scratch + kOffStart + i) = out; // lo and i are multiples of four
-		else
-			for (int q = 0; q < 4; q++)
-				if (i + q < hi)
-					scratch[kOffStart + i + q] = q == 0 ? out.x : q == 1 ? out.y : q == 2 ? out.z : out.w;
-#pragma unroll
-		for (int q = 0; q < 4; q++)
-			if (c[q] > kNaChain)
-				scratch[kOffBig + atomicAdd(scratch + kOffNbig, 1)] = i + q;
-		base += total;
-	}
-	if (!na_barrier(scratch))
-		return;
-
-	const bool once = n <= stride;
-	for (int i = t; i < n; i += stride)
-	{
-		if (!once)
-			key = voxel(i);
-		const int st = scratch[kOffStart + key], cnt = counts[key];
-		int j = scratch[kOffHead + key];
-		int rank = 0;
-		if (cnt > kNaChain)
-			for (rank = 0; j != i && rank + 1 < cnt; rank++) // its place on the chain
-				j = scratch[kOffNext + j];
-		else
-			for (int u = 0; u < cnt; u++)
+		if (threadIdx.x == 0)
+		{
+			const int q = next, phase = q / G;
+			s_next = q;
+			s_ok = phase == 0 || (phase < 5 && na_wait(words, min(phase, 3) * G, counts));
+		}
+		__syncthreads();
+		const int phase = s_next / G, item = s_next % G, t = item * kNaThreads + threadIdx.x;
+		if (!s_ok)
+			break;
+		if (phase == 0)
+		{
+			// the caller's buffer is 4-byte aligned at least
+			const int head = min(nvox, (int)((16 - (reinterpret_cast<uintptr_t>(counts) & 15)) & 15) / 4);
+			const int n4 = (nvox - head) / 4;
+			for (int k = t; k < n4; k += stride)
+				reinterpret_cast<int4*>(counts + head)[k] = make_int4(0, 0, 0, 0);
+			if (t < head)
+				counts[t] = 0;
+			if (t < nvox - head - 4 * n4)
+				counts[head + 4 * n4 + t] = 0;
+			if (t < G)
+				scratch[kOffTile + t] = 0;
+			if (t == 0)
 			{
-				rank += j > i;
-				if (u + 1 < cnt)
-					j = scratch[kOffNext + j];
+				scratch[kOffNbig] = 0;
+				if (after)
+					after->ticket = after->done = 0;
 			}
-		agents[st + rank] = i;
-	}
-	const int nbig = scratch[kOffNbig]; // the same for every block
-	if (nbig == 0 || !na_barrier(scratch))
-		return;
-	for (int b = blockIdx.x; b < nbig; b += gridDim.x)
-	{
-		const int v = scratch[kOffBig + b], st = scratch[kOffStart + v];
-		na_sort(agents + st, counts[v], scratch + kOffNext + st, sh);
+		}
+		else if (phase == 1)
+		{
+			for (int k = threadIdx.x; k < G; k += kNaThreads)
+				sh[k] = 0;
+			__syncthreads();
+			for (int i = t; i < n; i += stride)
+			{
+				const int c0 = na_axis(pos[(int64_t)i * m.dims], m, 0);
+				const int c1 = m.dims >= 2 ? na_axis(pos[(int64_t)i * m.dims + 1], m, 1) : 0;
+				const int c2 = m.dims >= 3 ? na_axis(pos[(int64_t)i * m.dims + 2], m, 2) : 0;
+				const int key = c0 + m.grid[0] * (c1 + m.grid[1] * c2);
+				atomicAdd(counts + key, 1);
+				const int before = atomicExch(scratch + kOffHead + key, i);
+				atomicAdd(sh + key / range, 1);
+				scratch[kOffKey + i] = key;
+				scratch[kOffNext + i] = before;
+			}
+			__syncthreads();
+			for (int k = threadIdx.x; k < G; k += kNaThreads)
+				if (sh[k])
+					atomicAdd(scratch + kOffTile + k, sh[k]);
+		}
+		else if (phase == 2)
+		{
+			int part = 0;
+			for (int k = threadIdx.x; k < item; k += kNaThreads)
+				part += scratch[kOffTile + k];
+			const int lo = item * range, hi = min(nvox, lo + range);
+			int c[4];
+			auto load = [&](int i) {
+#pragma unroll
+				for (int q = 0; q < 4; q++)
+					c[q] = i + q < hi ? counts[i + q] : 0;
+			};
+			load(lo + 4 * threadIdx.x);
+			int base;
+			na_block_scan(part, base);
+			for (int b = lo; b < hi; b += 4 * kNaThreads)
+			{
+				const int i = b + 4 * threadIdx.x;
+				if (b > lo)
+					load(i);
+				int total;
+				int4 out;
+				out.x = base + na_block_scan(c[0] + c[1] + c[2] + c[3], total);
+				out.y = out.x + c[0];
+				out.z = out.y + c[1];
+				out.w = out.z + c[2];
+				if (i + 3 < hi)
+					*reinterpret_cast<int4*>(scratch + kOffStart + i) = out; // lo and i are multiples of four
+				else
+					for (int q = 0; q < 4; q++)
+						if (i + q < hi)
+							scratch[kOffStart + i + q] = q == 0 ? out.x : q == 1 ? out.y : q == 2 ? out.z : out.w;
+#pragma unroll
+				for (int q = 0; q < 4; q++)
+					if (c[q] > kNaChain)
+						scratch[kOffBig + atomicAdd(scratch + kOffNbig, 1)] = i + q;
+				base += total;
+			}
+		}
+		else if (phase == 3)
+		{
+			for (int i = t; i < n; i += stride)
+			{
+				const int key = min((unsigned)scratch[kOffKey + i], (unsigned)(nvox - 1));
+				const int st = scratch[kOffStart + key], cnt = counts[key];
+				int j = scratch[kOffHead + key], rank = 0;
+				if (cnt > kNaChain)
+					for (; j != i && rank + 1 < cnt && (unsigned)j < (unsigned)n; rank++) // its place on the chain
+						j = scratch[kOffNext + j];
+				else
+					for (int u = 0; u < cnt && (unsigned)j < (unsigned)n; u++)
+					{
+						rank += j > i;
+						if (u + 1 < cnt)
+							j = scratch[kOffNext + j];
+					}
+				if ((unsigned)(st + rank) < (unsigned)n)
+					agents[st + rank] = i;
+			}
+		}
+		else
+		{
+			const int nbig = scratch[kOffNbig];
+			if (nbig == 0)
+				break; // the same for every block: set by the scan
+			if (threadIdx.x == 0)
+				s_all = na_wait(words, 4 * G, counts);
+			__syncthreads();
+			if (!s_all)
+				break;
+			for (int b = item; b < min(nbig, PPC_NOALLOC_MAX_AGENTS); b += G)
+			{
+				const int v = min((unsigned)scratch[kOffBig + b], (unsigned)(nvox - 1)), st = scratch[kOffStart + v];
+				if ((unsigned)st < (unsigned)n && counts[v] <= n - st)
+					na_sort(agents + st, counts[v], scratch + kOffNext + st, sh);
+			}
+		}
+		__syncthreads();
+		if (threadIdx.x == 0)
+		{
+			next = atomicAdd(&words->ticket, 1); // its way and that of the item's stores overlap
+			asm volatile("red.release.gpu.global.add.s32 [%0], 1;" ::"l"(&words->done) : "memory");
+		}
 	}
 }
 
 std::mutex g_na_mutex;
 void* g_na_ptr[256] = {};
 int g_na_blocks[256] = {}; // blocks of a whole grid, one per SM
+cudaEvent_t g_na_event[256] = {};			// the end of the device's last call...
+unsigned long long g_na_stream[256] = {}; // ...and one above the id of its stream (0: none yet)
+int g_na_set[256] = {};					  // words of the next call
 
 } // namespace
 
@@ -373,44 +415,60 @@ extern "C" int ppc_bin_agents_noalloc(const ppc_mesh* mesh, const double* positi
 	cudaError_t e = cudaGetDevice(&dev);
 	if (e != cudaSuccess || dev < 0 || dev >= 256)
 		return e != cudaSuccess ? ppc::cuda_fail(e, "cudaGetDevice") : PPC_ERR_NO_DEVICE;
-	int32_t* scratch = nullptr;
-	int blocks = 1;
-	{
-		std::lock_guard<std::mutex> lock(g_na_mutex);
-		if (!g_na_ptr[dev])
-		{
-			int per_sm = 0, sms = 0;
-			e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_na_bins, kNaThreads, 0);
-			if (e == cudaSuccess)
-				e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-			if (e != cudaSuccess || per_sm < 1)
-				return ppc::cuda_fail(e != cudaSuccess ? e : cudaErrorInvalidConfiguration, "k_na_bins");
-			g_na_blocks[dev] = std::min(sms, (int)kNaBlocks);
-			void* p = nullptr;
-			e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
-			if (e != cudaSuccess)
-				return ppc::cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
-			g_na_ptr[dev] = p;
-		}
-		scratch = static_cast<int32_t*>(g_na_ptr[dev]);
-		blocks = g_na_blocks[dev];
-	}
-
 	cudaStream_t st = static_cast<cudaStream_t>(cuda_stream);
 	if (count == 0)
 	{
 		PPC_CUDA(cudaMemsetAsync(voxel_counts, 0, sizeof(int32_t) * nvox, st));
 		return PPC_OK;
 	}
-	cudaLaunchConfig_t cfg {};
-	cfg.gridDim = dim3(std::min(blocks, std::max((count + kNaThreads - 1) / kNaThreads, (int)(nvox / (4 * kNaThreads)) + 1)));
-	cfg.blockDim = dim3(kNaThreads);
-	cfg.stream = st;
-	cudaLaunchAttribute at[1];
-	at[0].id = cudaLaunchAttributeCooperative;
-	at[0].val.cooperative = 1;
-	cfg.attrs = at;
-	cfg.numAttrs = 1;
-	PPC_CUDA(cudaLaunchKernelEx(&cfg, k_na_bins, positions, count, m, voxel_counts, scratch, agents));
+	std::lock_guard<std::mutex> lock(g_na_mutex);
+	if (!g_na_ptr[dev])
+	{
+		int sms = 0;
+		e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+		if (e == cudaSuccess && !g_na_event[dev])
+			e = cudaEventCreateWithFlags(&g_na_event[dev], cudaEventDisableTiming);
+		if (e != cudaSuccess)
+			return ppc::cuda_fail(e, "ppc_bin_agents_noalloc");
+		g_na_blocks[dev] = std::min(sms, kNaBlocks);
+		void* p = nullptr;
+		e = cudaGetSymbolAddress(&p, g_noalloc_scratch);
+		if (e != cudaSuccess)
+			return ppc::cuda_fail(e, "cudaGetSymbolAddress(g_noalloc_scratch)");
+		g_na_ptr[dev] = p;
+	}
+	int32_t* scratch = static_cast<int32_t*>(g_na_ptr[dev]);
+	na_words* const sets = reinterpret_cast<na_words*>(scratch + kOffWords);
+	na_words *words = sets + g_na_set[dev], *after = sets + (g_na_set[dev] ^ 1);
+	const int blocks
+		= std::min(g_na_blocks[dev], std::max((count + kNaThreads - 1) / kNaThreads, (int)(nvox / (4 * kNaThreads)) + 1));
+
+	// a captured call has words of its own, cleared in the graph; others wait
+	// for the call before them where that was on another stream
+	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(st, &cs) != cudaSuccess)
+		cudaGetLastError(); // the launch reports it
+	const bool captured = cs != cudaStreamCaptureStatusNone;
+	unsigned long long id = 0;
+	if (captured)
+	{
+		words = sets + 2;
+		after = nullptr;
+		PPC_CUDA(cudaMemsetAsync(words, 0, sizeof(na_words), st));
+	}
+	else
+	{
+		PPC_CUDA(cudaStreamGetId(st, &id));
+		if (g_na_stream[dev] != 0 && g_na_stream[dev] != id + 1)
+			PPC_CUDA(cudaStreamWaitEvent(st, g_na_event[dev], 0));
+	}
+	k_na_bins<<<blocks, kNaThreads, 0, st>>>(positions, count, m, voxel_counts, scratch, words, after, agents);
+	PPC_CUDA(cudaGetLastError());
+	if (!captured)
+	{
+		g_na_set[dev] ^= 1;
+		PPC_CUDA(cudaEventRecord(g_na_event[dev], st));
+		g_na_stream[dev] = id + 1;
+	}
 	return PPC_OK;
 }

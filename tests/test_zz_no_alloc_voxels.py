@@ -42,3 +42,79 @@ def test_crowded_voxels(clump, spread, side, shift):
         assert np.array_equal(counts.cpu().numpy()[shift:], want_counts)
         assert np.array_equal(agents.cpu().numpy()[shift:], want_agents)
         assert (counts[:shift] == -7).all() and (agents[:shift] == -7).all()
+
+
+def _case(n, side, seed):
+    import torch
+
+    rng = np.random.default_rng(seed)
+    pos = rng.random((n, 3)) * 30 * side
+    key = (pos / 30.0).astype(np.int64)
+    key = key[:, 0] + side * (key[:, 1] + side * key[:, 2])
+    return {"mesh": Mesh.make(3, (0, 0, 0), (30 * side,) * 3), "n": n, "pos": torch.from_numpy(pos.ravel()).cuda(),
+            "counts": torch.full((side ** 3,), -7, dtype=torch.int32, device="cuda"),
+            "agents": torch.full((n,), -7, dtype=torch.int32, device="cuda"),
+            "want": (np.bincount(key, minlength=side ** 3), np.lexsort((-np.arange(n), key)))}
+
+
+def _call(L, c, stream):
+    rc = L.ppc_bin_agents_noalloc(C.byref(c["mesh"]), c["pos"].data_ptr(), c["n"], c["counts"].data_ptr(),
+                                  c["agents"].data_ptr(), stream.cuda_stream)
+    assert rc == 0, L.ppc_last_error()
+
+
+def _check(c):
+    assert np.array_equal(c["counts"].cpu().numpy(), c["want"][0])
+    assert np.array_equal(c["agents"].cpu().numpy(), c["want"][1])
+    c["counts"].fill_(-7)
+    c["agents"].fill_(-7)
+
+
+def _lib():
+    from paraphysicell_b200 import device
+
+    build.ensure_built()
+    L = device.lib()
+    L.ppc_bin_agents_noalloc.argtypes = [C.POINTER(Mesh), C.c_void_p, C.c_int32, C.c_void_p, C.c_void_p, C.c_void_p]
+    return L
+
+
+def test_calls_on_two_streams_run_one_after_another():
+    """Calls of different grids queued on two streams without a wait between
+    them, and calls after them."""
+    import torch
+
+    L = _lib()
+    cases = [_case(131072, 101, 1), _case(700, 5, 2), _case(20000, 9, 3), _case(1, 3, 4)]
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    torch.cuda.synchronize()
+    for r in range(3):
+        for k, c in enumerate(cases):
+            _call(L, c, streams[(k + r) % 2])
+        torch.cuda.synchronize()
+        for c in cases:
+            _check(c)
+        torch.cuda.synchronize()
+
+
+def test_captured_call_replays():
+    import torch
+
+    L = _lib()
+    c, other = _case(30000, 30, 5), _case(4000, 4, 6)
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    _call(L, c, stream)
+    torch.cuda.synchronize()
+    _check(c)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=stream):
+        _call(L, c, torch.cuda.current_stream())
+    for _ in range(3):
+        graph.replay()
+        torch.cuda.synchronize()
+        _check(c)
+        _call(L, other, torch.cuda.current_stream())
+        torch.cuda.synchronize()
+        _check(other)
+        torch.cuda.synchronize()
