@@ -579,9 +579,10 @@ int ppc_get_profile(ppc_state* s, double* fused_ms, int64_t* fused_launches);
  * agents grouped by voxel, descending index inside a voxel. Scratch lives in
  * one fixed device array; sizes above PPC_NOALLOC_MAX_AGENTS or
  * PPC_NOALLOC_MAX_VOXELS return PPC_ERR_CAPACITY (the grid is sized in 64-bit
- * arithmetic, so no mesh extent can wrap it). The in-voxel ordering pass costs
- * c^2 loads for a voxel of c agents: negligible at tissue densities, about a
- * second of GPU time if all PPC_NOALLOC_MAX_AGENTS agents share one voxel. Nothing is allocated. The first call on a device
+ * arithmetic, so no mesh extent can wrap it). The in-voxel order of a voxel
+ * of more than 24 agents costs c^2 loads for its c agents: negligible at
+ * tissue densities, about 3.4 ms of GPU time if all PPC_NOALLOC_MAX_AGENTS
+ * agents share one voxel. Nothing is allocated. The first call on a device
  * looks the array's address up for that device, so make that first call
  * before any stream capture. All calls on a device share the array: calls on
  * different streams run one after another (an event orders them), but graph

@@ -33,19 +33,19 @@ namespace {
 
 constexpr int kNaThreads = 1024;
 constexpr int kNaBlocks = 1024; // more than any grid has
-constexpr int kNaChain = 24; // agents of a voxel whose order their chain gives; larger voxels are sorted by a block
-constexpr int kNaSort = 4096; // agents of one voxel sorted in shared memory
+constexpr int kNaChain = 24;	// agents of a voxel whose order their chain gives; those of larger ones are compared
 constexpr int kNaWait = 1 << 22; // polls of a wait before it gives up, about two seconds
 
 // layout of the scratch, in int32 units
 constexpr int64_t kOffNext = 0;
 constexpr int64_t kOffKey = kOffNext + PPC_NOALLOC_MAX_AGENTS;
-constexpr int64_t kOffBig = kOffKey + PPC_NOALLOC_MAX_AGENTS; // voxels whose agents a block sorts
-constexpr int64_t kOffHead = kOffBig + PPC_NOALLOC_MAX_AGENTS;
+constexpr int64_t kOffRank = kOffKey + PPC_NOALLOC_MAX_AGENTS;
+constexpr int64_t kOffTmp = kOffRank + PPC_NOALLOC_MAX_AGENTS;
+constexpr int64_t kOffHead = kOffTmp + PPC_NOALLOC_MAX_AGENTS;
 constexpr int64_t kOffStart = kOffHead + PPC_NOALLOC_MAX_VOXELS;
 constexpr int64_t kOffTile = kOffStart + PPC_NOALLOC_MAX_VOXELS;
-constexpr int64_t kOffNbig = kOffTile + kNaBlocks;
-constexpr int64_t kOffWords = kOffNbig + 32; // na_words: two that calls use in turn, and the captured calls'
+constexpr int64_t kOffBig = kOffTile + kNaBlocks; // a voxel has more than kNaChain agents
+constexpr int64_t kOffWords = kOffBig + 32; // na_words: two that calls use in turn, and the captured calls'
 constexpr int64_t kWordsInts = 2 * 32;
 constexpr int64_t kScratchInts = kOffWords + 3 * kWordsInts;
 
@@ -133,55 +133,8 @@ __device__ __forceinline__ int na_block_scan(int x, int& total)
 	return excl;
 }
 
-// Sorts the `c` agents of a large voxel, at `agents`, by one block: a bitonic
-// sort in shared memory, or for more than kNaSort agents rank counting over a
-// copy. Tissue has no such voxel.
-__device__ void na_sort(int32_t* agents, int c, int32_t* copy, int32_t* sh)
-{
-	if (c <= kNaSort)
-	{
-		int m = 1;
-		while (m < c)
-			m <<= 1;
-		for (int u = threadIdx.x; u < m; u += kNaThreads)
-			sh[u] = u < c ? agents[u] : -1;
-		__syncthreads();
-		for (int k = 2; k <= m; k <<= 1)
-			for (int h = k >> 1; h > 0; h >>= 1)
-			{
-				for (int u = threadIdx.x; u < m; u += kNaThreads)
-				{
-					const int l = u ^ h;
-					if (l > u && (sh[u] < sh[l]) == ((u & k) == 0))
-					{
-						const int x = sh[u];
-						sh[u] = sh[l];
-						sh[l] = x;
-					}
-				}
-				__syncthreads();
-			}
-		for (int u = threadIdx.x; u < c; u += kNaThreads)
-			agents[u] = sh[u];
-		__syncthreads();
-		return;
-	}
-	for (int u = threadIdx.x; u < c; u += kNaThreads)
-		copy[u] = agents[u];
-	__syncthreads();
-	for (int u = threadIdx.x; u < c; u += kNaThreads)
-	{
-		const int x = copy[u];
-		int rank = 0;
-		for (int w = 0; w < c; w++)
-			rank += copy[w] > x;
-		agents[rank] = x;
-	}
-	__syncthreads();
-}
-
 // The whole call as one launch. The phases clear, count, scan, place and
-// sort have an item per block each. A block takes the items in their order
+// compare have an item per block each. A block takes the items in their order
 // off a counter, whatever its index, and an item starts once every item of the
 // phases before is done. So an item waits only for items that blocks already
 // running have taken: the launch needs no set of blocks resident at once, and
@@ -192,18 +145,21 @@ __device__ void na_sort(int32_t* agents, int c, int32_t* copy, int32_t* sh)
 // dependent phases: a memset and five launches take 34.2 us, one
 // launch with grid barriers (which needs all its blocks resident) 20.5, this one
 // 20.6 to 21.2 us.
-//  count: an agent's voxel, and its link on the voxel's chain. The chain's
-//   last link is whatever the scratch held: whoever walks it knows the count.
-//   The totals of the blocks' voxel ranges are formed here too.
+//  count: an agent's voxel, its number there, and its link on the voxel's
+//   chain. The chain's last link is whatever the scratch held: whoever walks it
+//   knows the count. The totals of the blocks' voxel ranges are formed here too.
 //  scan: the starts of a range of voxels.
-//  place: descending index inside the voxel, from the agents on its chain; an
-//   agent of a voxel of more than kNaChain takes its place on the chain, and a
-//   block sorts the voxel in the last phase.
+//  place: descending index inside the voxel, from the agents on its chain.
+//   Agents of a voxel of more than kNaChain are gathered by their numbers and
+//   compare with one another in the last phase: c^2 loads for c agents, as
+//   many as the grid's threads at once. All 131,072 in one voxel take 3.4 ms
+//   (a walk along the chain and a block's sort: 380 ms), 3,000 voxels of 30
+//   among 31,000 agents 33 us (110 us).
 __global__ void __launch_bounds__(kNaThreads, 1)
 	k_na_bins(const double* __restrict__ pos, int n, na_mesh m, int32_t* counts, int32_t* scratch, na_words* words,
 			  na_words* after, int32_t* agents)
 {
-	__shared__ int32_t sh[kNaSort];
+	__shared__ int32_t sh[kNaBlocks];
 	__shared__ int s_next, s_ok, s_all;
 	const int G = gridDim.x, stride = G * kNaThreads;
 	const int nvox = m.nvox;
@@ -239,7 +195,7 @@ __global__ void __launch_bounds__(kNaThreads, 1)
 				scratch[kOffTile + t] = 0;
 			if (t == 0)
 			{
-				scratch[kOffNbig] = 0;
+				scratch[kOffBig] = 0;
 				if (after)
 					after->ticket = after->done = 0;
 			}
@@ -255,10 +211,11 @@ __global__ void __launch_bounds__(kNaThreads, 1)
 				const int c1 = m.dims >= 2 ? na_axis(pos[(int64_t)i * m.dims + 1], m, 1) : 0;
 				const int c2 = m.dims >= 3 ? na_axis(pos[(int64_t)i * m.dims + 2], m, 2) : 0;
 				const int key = c0 + m.grid[0] * (c1 + m.grid[1] * c2);
-				atomicAdd(counts + key, 1);
+				const int number = atomicAdd(counts + key, 1);
 				const int before = atomicExch(scratch + kOffHead + key, i);
 				atomicAdd(sh + key / range, 1);
 				scratch[kOffKey + i] = key;
+				scratch[kOffRank + i] = number;
 				scratch[kOffNext + i] = before;
 			}
 			__syncthreads();
@@ -298,10 +255,8 @@ __global__ void __launch_bounds__(kNaThreads, 1)
 					for (int q = 0; q < 4; q++)
 						if (i + q < hi)
 							scratch[kOffStart + i + q] = q == 0 ? out.x : q == 1 ? out.y : q == 2 ? out.z : out.w;
-#pragma unroll
-				for (int q = 0; q < 4; q++)
-					if (c[q] > kNaChain)
-						scratch[kOffBig + atomicAdd(scratch + kOffNbig, 1)] = i + q;
+				if (max(max(c[0], c[1]), max(c[2], c[3])) > kNaChain)
+					scratch[kOffBig] = 1;
 				base += total;
 			}
 		}
@@ -311,36 +266,45 @@ __global__ void __launch_bounds__(kNaThreads, 1)
 			{
 				const int key = min((unsigned)scratch[kOffKey + i], (unsigned)(nvox - 1));
 				const int st = scratch[kOffStart + key], cnt = counts[key];
-				int j = scratch[kOffHead + key], rank = 0;
 				if (cnt > kNaChain)
-					for (; j != i && rank + 1 < cnt && (unsigned)j < (unsigned)n; rank++) // its place on the chain
+				{
+					const int at = st + scratch[kOffRank + i];
+					if ((unsigned)at < (unsigned)n)
+						scratch[kOffTmp + at] = i;
+					continue;
+				}
+				int j = scratch[kOffHead + key], rank = 0;
+				for (int u = 0; u < cnt && (unsigned)j < (unsigned)n; u++)
+				{
+					rank += j > i;
+					if (u + 1 < cnt)
 						j = scratch[kOffNext + j];
-				else
-					for (int u = 0; u < cnt && (unsigned)j < (unsigned)n; u++)
-					{
-						rank += j > i;
-						if (u + 1 < cnt)
-							j = scratch[kOffNext + j];
-					}
+				}
 				if ((unsigned)(st + rank) < (unsigned)n)
 					agents[st + rank] = i;
 			}
 		}
 		else
 		{
-			const int nbig = scratch[kOffNbig];
-			if (nbig == 0)
+			if (scratch[kOffBig] == 0)
 				break; // the same for every block: set by the scan
 			if (threadIdx.x == 0)
 				s_all = na_wait(words, 4 * G, counts);
 			__syncthreads();
 			if (!s_all)
 				break;
-			for (int b = item; b < min(nbig, PPC_NOALLOC_MAX_AGENTS); b += G)
+			// warp by warp over the items, so that all of them have the same share
+			for (int i = ((threadIdx.x >> 5) * G + item) * 32 + (threadIdx.x & 31); i < n; i += stride)
 			{
-				const int v = min((unsigned)scratch[kOffBig + b], (unsigned)(nvox - 1)), st = scratch[kOffStart + v];
-				if ((unsigned)st < (unsigned)n && counts[v] <= n - st)
-					na_sort(agents + st, counts[v], scratch + kOffNext + st, sh);
+				const int key = min((unsigned)scratch[kOffKey + i], (unsigned)(nvox - 1));
+				const int st = scratch[kOffStart + key], cnt = counts[key];
+				if (cnt <= kNaChain || (unsigned)st >= (unsigned)n || cnt > n - st)
+					continue;
+				const int32_t* all = scratch + kOffTmp + st;
+				int rank = 0;
+				for (int u = 0; u < cnt; u++)
+					rank += all[u] > i;
+				agents[st + rank] = i;
 			}
 		}
 		__syncthreads();

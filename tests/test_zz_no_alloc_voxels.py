@@ -118,3 +118,27 @@ def test_captured_call_replays():
         torch.cuda.synchronize()
         _check(other)
         torch.cuda.synchronize()
+
+
+def test_all_agents_in_one_voxel():
+    """131,072 agents in the middle one of 27 voxels: compared by the whole
+    grid in some 3.4 ms. A walk along the voxel's chain takes 380 ms; the bound
+    lies a factor of ten from both."""
+    import torch
+
+    L = _lib()
+    c = _case(131072, 3, 7)
+    c["pos"].copy_(30.0 + c["pos"] / 3.0)
+    counts = np.zeros(27, np.int64)
+    counts[13] = c["n"]
+    c["want"] = (counts, np.arange(c["n"])[::-1])
+    stream = torch.cuda.current_stream()
+    _call(L, c, stream)
+    _check(c)
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    _call(L, c, stream)
+    b.record()
+    torch.cuda.synchronize()
+    _check(c)
+    assert a.elapsed_time(b) < 35.0
