@@ -208,11 +208,12 @@ enum ppc_step_form
 };
 int ppc_set_step_form(ppc_state* s, int32_t form);
 
-/* Bound of every device-side wait (the persistent step's grid barriers), in
- * polls of about 64 ns each; the default 2^25 is about two seconds. A wait
- * that runs out leaves the step incomplete: the next synchronising call
- * returns PPC_ERR_TIMEOUT, later persistent steps do nothing until then, and
- * ppc_step refuses to run until the state is uploaded again. */
+/* Bound of every wait of a step's grid barriers (steps over neighbour lists,
+ * persistent steps), in polls of a few hundred nanoseconds each (a load's way
+ * to the L2 and back); the default 2^25 is some ten seconds. A wait that runs
+ * out leaves the step incomplete: the next synchronising call returns
+ * PPC_ERR_TIMEOUT, later such steps do nothing until then, and ppc_step
+ * refuses to run until the state is uploaded again. */
 int ppc_set_wait_limit(ppc_state* s, int64_t polls);
 
 /* Autotuner of the launch shape (no counterpart in the reference, whose

@@ -260,8 +260,7 @@ int map_errors(ppc_state* s, int32_t err)
 	if (err & ERR_TIMEOUT)
 	{
 		s->lost = true;
-		return fail(PPC_ERR_TIMEOUT, "a grid barrier of the persistent step gave up waiting; the state must be "
-									 "uploaded again");
+		return fail(PPC_ERR_TIMEOUT, "a grid barrier of a step gave up waiting; the state must be uploaded again");
 	}
 	if (err & ERR_NONFINITE)
 		return fail(PPC_ERR_NONFINITE, "an agent position is NaN or infinite");
@@ -1531,6 +1530,35 @@ int ppc_set_neighbor_capacity(ppc_state* s, int32_t per_agent)
 	return PPC_OK;
 }
 
+} // extern "C"
+
+namespace ppc {
+namespace {
+
+// What a step left that gave up at a barrier: arrivals at the barriers, movers
+// on the tiles' chains, planned moves, and removal candidates.
+int reset_interrupted(ppc_state* s)
+{
+	const view& v = s->v;
+	const size_t C = s->total_cap, tiles = v.ntiles, word = sizeof(int32_t);
+	if (s->lists_fit)
+		PPC_CUDA(cudaMemsetAsync(s->list_bar, 0, 64 * sizeof(unsigned long long), s->stream));
+	PPC_CUDA(cudaMemsetAsync(v.chead, 0xff, 32 * tiles * word, s->stream));
+	PPC_CUDA(cudaMemsetAsync(v.tdelta, 0, tiles * word, s->stream));
+	PPC_CUDA(cudaMemsetAsync(v.sdelta, 0, (tiles + 1023) / 1024 * word, s->stream));
+	PPC_CUDA(cudaMemsetAsync(v.move_src, 0xff, C * word, s->stream));
+	for (int32_t* flag : { v.moves_pending, v.appended, v.recount })
+		PPC_CUDA(cudaMemsetAsync(flag, 0, word, s->stream));
+	for (int32_t r = 0; r < s->nreps; r++)
+		PPC_CUDA(cudaMemsetAsync(&v.ctr[r].nbad, 0, word, s->stream));
+	return PPC_OK;
+}
+
+} // namespace
+} // namespace ppc
+
+extern "C" {
+
 int ppc_upload(ppc_state* s, int32_t r, const ppc_agents* a)
 {
 	if (!valid(s, r) || !a || a->count < 0)
@@ -1549,8 +1577,8 @@ int ppc_upload(ppc_state* s, int32_t r, const ppc_agents* a)
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
 	s->lists_stale = false;
 	s->skin_reset = true;
-	if (s->lost && s->lists_fit)
-		PPC_CUDA(cudaMemsetAsync(s->list_bar, 0, 64 * sizeof(unsigned long long), s->stream));
+	if (s->lost)
+		PPC_TRY(reset_interrupted(s));
 	s->lost = false;
 	return transfer_in(s, r, a, true);
 }

@@ -4625,7 +4625,7 @@ static int list_launch(ppc_state* s, const list_args& a)
 int launch_list_steps(ppc_state* s, int steps)
 {
 	list_args a {};
-	a.limit = 1LL << 25; // about 20 s of polls
+	a.limit = s->wait_limit;
 	a.opts = fused_opts(s);
 	a.steps = steps;
 	a.p = s->lcur;

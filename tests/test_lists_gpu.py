@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 from paraphysicell_b200 import workloads as wl
-from paraphysicell_b200.abi import AgentArrays, Mesh, Params
+from paraphysicell_b200.abi import PPC_ERR_ARG, PPC_ERR_TIMEOUT, AgentArrays, Mesh, Params, PPCError
 
 from tests.gpu_util import assert_same_bins, assert_same_state, fetch, make_pair
 
@@ -174,6 +174,28 @@ def test_two_live_states_of_different_capacity(capacities):
             assert_same_state(fetch(d, a), fetch(o, a))
     for o, d, a in pairs:
         d.close()
+
+
+@pytest.mark.parametrize("form", FORMS)
+def test_barrier_timeout_is_reported_and_recoverable(form):
+    """A one-poll wait limit makes the grid barriers of a call over lists give
+    up: PPC_ERR_TIMEOUT at the next synchronising call, steps refused until the
+    state is uploaded again, and from then on the oracle's trajectory."""
+    mesh, params, a = _agents(3000, 3, 150, 51, FORMS[form], fast=20.0)
+    o, d = make_pair(mesh, params, a)
+    d.step(5)
+    d.set_wait_limit(1)
+    d.step(60)
+    with pytest.raises(PPCError) as e:
+        d.synchronize()
+    assert e.value.rc == PPC_ERR_TIMEOUT
+    with pytest.raises(PPCError) as e:
+        d.step(4)
+    assert e.value.rc == PPC_ERR_ARG
+    d.set_wait_limit(1 << 25)
+    d.upload(a)
+    _run(o, d, a, (5, 12, 1, 9))
+    d.close()
 
 
 def test_fp32_force_lists_match_the_scanning_pass():
