@@ -2170,32 +2170,31 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 	}
 	else if (!s->ix_store.p)
 		return fail(PPC_ERR_ARG, "no resident interaction fields: upload them or pass fields");
-	const int32_t n = most_rows(s, r); // known where the fields came with the call
+	// The scratch has a row per live agent and some to spare. Where the host
+	// does not know the count the pass runs over the rows there are, and does
+	// nothing if the agents are more.
+	const size_t row = sizeof(int32_t) * (4 + (size_t)s->ncap);
+	int32_t n = (int32_t)std::min<size_t>(s->ix_scratch_bytes / row, s->reps[r].cap);
+	if (s->counts_known) // also where the fields came with the call
+		n = s->host_count[r];
+	else if (n == 0)
+		PPC_TRY(live_count(s, r, n));
 	if ((int32_t)s->ix_epoch.size() < s->nreps)
 		s->ix_epoch.resize(s->nreps, 0);
 	const uint64_t epoch = s->ix_epoch[r]++;
 	if (n == 0)
 		return PPC_OK;
 	PPC_TRY(ensure_lists(s));
-	const size_t nd = (size_t)n;
-	PPC_TRY(ensure_field_scratch(s, sizeof(int32_t) * (4 * nd + nd * s->ncap)));
-	int32_t* ip = static_cast<int32_t*>(s->ix_scratch);
 	const int32_t base = s->reps[r].base;
 	const ix_columns& c = s->v.ix;
 	const size_t D = s->ndefs, S = c.S;
 	ix_fields x {};
-	x.n = n;
 	x.substrates = c.S;
 	x.replicate = r;
 	x.base = base;
 	x.dt = s->params.mechanics_time_step;
 	x.epoch = epoch;
 	x.status = s->v.err + 1; // the words after the error word, spare
-	x.ncand = ip;
-	x.dep = ip + nd;
-	x.walk = ip + 2 * nd;
-	x.order = ip + 3 * nd;
-	x.cand = ip + 4 * nd;
 	x.dead = c.dead + base;
 	x.dead_phago = c.dead_phago + base;
 	x.damage_rate = c.damage_rate + base;
@@ -2219,10 +2218,25 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 	x.target_cyto = c.target_cyto + base;
 	x.target_nuc = c.target_nuc + base;
 	x.isub = c.isub + base * S;
-	PPC_CUDA(cudaMemsetAsync(x.status, 0, 3 * sizeof(int32_t), s->stream));
-	PPC_TRY(launch_interactions(s, x));
-	// the call's status, the device error word and the counts in one copy
-	PPC_TRY(finish_counts(s));
+	for (;; n = s->host_count[r])
+	{
+		if (n * row > s->ix_scratch_bytes)
+			PPC_TRY(ensure_field_scratch(s, row * std::min<int64_t>(s->reps[r].cap, (int64_t)n + n / 8 + 1024)));
+		int32_t* ip = static_cast<int32_t*>(s->ix_scratch);
+		const size_t nd = (size_t)n;
+		x.n = n;
+		x.ncand = ip;
+		x.dep = ip + nd;
+		x.walk = ip + 2 * nd;
+		x.order = ip + 3 * nd;
+		x.cand = ip + 4 * nd;
+		PPC_CUDA(cudaMemsetAsync(x.status, 0, 3 * sizeof(int32_t), s->stream));
+		PPC_TRY(launch_interactions(s, x));
+		// the call's status, the device error word and the counts in one copy
+		PPC_TRY(finish_counts(s));
+		if (!(s->pinned_err[1] & 2))
+			break;
+	}
 	if (s->pinned_err[1])
 		return fail(PPC_ERR_CAPACITY, "a neighbour list exceeds the neighbour capacity: no interaction ran");
 	// positions and radii may have changed: the next mesh update rebuilds the
@@ -2235,7 +2249,7 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t r, ppc_interactions*
 		std::vector<column> back;
 		for (const auto& col : ix_column_list(s->v.ix, f, s->ndefs))
 			back.push_back(col);
-		PPC_TRY(move_columns(s, back, base, n, false));
+		PPC_TRY(move_columns(s, back, base, s->host_count[r], false));
 		return finish(s);
 	}
 	return map_errors(s, s->pinned_err[0]);

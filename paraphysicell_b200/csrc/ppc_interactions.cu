@@ -46,6 +46,12 @@ __global__ void __launch_bounds__(kIxThreads) k_ix_candidates(view v, ix_fields 
 {
 	const int i = blockIdx.x * blockDim.x + threadIdx.x;
 	const int n = v.ctr[x.replicate].count;
+	if (n > x.n)
+	{
+		if (i == 0)
+			atomicOr(x.status, 2); // the scratch has too few rows: nobody walks
+		return;
+	}
 	if (i >= n)
 		return;
 	int m = 0;

@@ -463,7 +463,7 @@ int launch_springs_local(ppc_state* s, int32_t r, int32_t n, int32_t* rows, int3
 // device copies of the ppc_interactions fields of one replicate (local rows)
 struct ix_fields
 {
-	int32_t n; // rows at most; the device's count says how many
+	int32_t n; // rows of the scratch; the device's count says how many live
 	int32_t substrates, replicate, base;
 	double dt;
 	uint64_t epoch;
@@ -475,7 +475,7 @@ struct ix_fields
 		*target_nuc, *isub;
 	int32_t* ncand; // [n] candidate neighbours of each agent
 	int32_t* cand;	// [n*ncap] their positions in the agent's neighbour list
-	int32_t* status; // [3] capacity error found by the candidate pass, agents that walk, agents left for the ordered pass
+	int32_t* status; // [3] errors found by the candidate pass (1: a cut list, 2: too few rows), agents that walk, agents left for the ordered pass
 	int32_t* walk;	 // [n] the agents with a candidate
 	int32_t* dep;	 // [n] 1 while a dependent agent has not walked
 	int32_t* order;	 // [n] the dependent agents still to walk

@@ -101,6 +101,36 @@ def test_interactions_leave_the_next_step_a_current_mesh(scale):
     d.close()
 
 
+def test_interaction_scratch_follows_the_live_agents():
+    """A state of 400,000 slots and 300 agents allocates rows for its agents,
+    not its slots (109 MB of them), and more once divisions outgrow them."""
+    import torch
+
+    mesh, params, a = wl.scaled(wl.config2, 300, seed=7, capacity=400000)
+    f = sc.random_interaction_fields(a, params.cell_definitions_count, seed=8, scale=0.02)
+    o, d = gu.make_pair(mesh, params, a)
+    _start(o, d)
+    for x in (o, d):
+        x.upload_interactions(f.copy())
+    free = torch.cuda.mem_get_info()[0]
+    d.update_mechanics_mesh()
+    for p_divide in (0.0, 0.9, 0.9, 0.9):
+        o.step(1, 1, p_divide, 0.0)
+        d.step_with_phenotype(1, p_divide, 0.0)
+        for x in (o, d):
+            x.update_mechanics_mesh()
+            x.update_cell_neighbors()
+        o.update_cell_cell_interactions()
+        d.update_cell_cell_interactions()
+        if p_divide == 0.0:
+            assert free - torch.cuda.mem_get_info()[0] < 16 << 20
+        gu.assert_same_state(gu.fetch(d, a), gu.fetch(o, a))
+        o.update_mechanics_mesh()  # the oracle's step starts from the lists it has
+        o.update_cell_neighbors()
+    assert d.count() > 300 + 300 // 8 + 1024
+    d.close()
+
+
 @pytest.mark.parametrize("n", [131071, 131072, 300001])
 def test_large_downloads_into_pageable_rows(n):
     """Columns at the landing area's threshold and beyond its size, and agents
