@@ -199,47 +199,37 @@ bool pull_column(ppc_state* s, void* dst, const void* src, size_t bytes, int wid
 	return true;
 }
 
-// Queues a device-to-host copy on the stream. The driver copies into pageable
-// memory with one thread, 5.5 GB/s; a large copy lands in the state's
-// page-locked area instead and drain_host, after the next synchronisation,
-// spreads the host copy over a few threads. 1 M agents, 72 MB of them 16 MB
-// pageable: 4.0 and 2.1 ms (of it: agents appended since the
-// last count no longer cost a second download of all).
+// Queues a device-to-host copy on the stream. Into pageable rows the driver
+// copies with one thread, which the host waits for. Where page-locked vectors
+// follow (s->landing), a large column lands in the state's page-locked area
+// instead, as long as there is room, and drain_host copies it on with a few
+// threads beside the vectors' transfer: 1 M agents, ten dividing steps and
+// 72 MB, 16 MB of them pageable, 5.33 ms with the driver's copies, 5.06 ms so.
+// With nothing to run beside, the driver is the faster one: all fields of
+// 300,000 agents into pageable rows 5.4 ms, through the area 15 ms.
 int copy_down(ppc_state* s, void* dst, const void* src, size_t bytes)
 {
+	void* to = dst;
 	cudaPointerAttributes at {};
-	const bool large = s->bounce && bytes >= kBounceLeast;
-	if (large && cudaPointerGetAttributes(&at, dst) != cudaSuccess)
-		cudaGetLastError();
-	if (!large || at.type != cudaMemoryTypeUnregistered)
+	if (s->landing && bytes >= kBounceLeast && bytes <= s->bounce_bytes - s->bounce_used)
 	{
-		PPC_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s->stream));
-		return PPC_OK;
-	}
-	while (bytes)
-	{
-		if (s->bounce_used == s->bounce_bytes)
+		if (cudaPointerGetAttributes(&at, dst) != cudaSuccess)
+			cudaGetLastError();
+		if (at.type == cudaMemoryTypeUnregistered)
 		{
-			PPC_CUDA(cudaStreamSynchronize(s->stream));
-			drain_host(s);
+			to = static_cast<char*>(s->bounce) + s->bounce_used;
+			s->pending_host.push_back({ dst, to, bytes });
+			s->bounce_used += bytes;
 		}
-		const size_t n = std::min(bytes, s->bounce_bytes - s->bounce_used);
-		char* land = static_cast<char*>(s->bounce) + s->bounce_used;
-		PPC_CUDA(cudaMemcpyAsync(land, src, n, cudaMemcpyDeviceToHost, s->stream));
-		s->pending_host.push_back({ dst, land, n });
-		s->bounce_pieces++;
-		s->bounce_used += n;
-		dst = static_cast<char*>(dst) + n;
-		src = static_cast<const char*>(src) + n;
-		bytes -= n;
 	}
+	PPC_CUDA(cudaMemcpyAsync(to, src, bytes, cudaMemcpyDeviceToHost, s->stream));
 	return PPC_OK;
 }
 
 int flush_copies(ppc_state* s)
 {
 	for (const auto& c : s->pending_copies)
-		PPC_TRY(copy_down(s, c.dst, c.src, c.bytes));
+		PPC_CUDA(cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, s->stream));
 	s->pending_copies.clear();
 	return PPC_OK;
 }
@@ -666,13 +656,27 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 	return PPC_OK;
 }
 
+// whether a download queues copies into vectors, all of them page-locked
+bool vectors_page_locked(const ppc_agents* a)
+{
+	bool any = false;
+	for (const double* p : { a->positions, a->velocities, a->previous_velocities, a->orientation })
+	{
+		if (p && !mapped(p))
+			return false;
+		any = any || p;
+	}
+	return any;
+}
+
 // queues the copies of agents [first, n) of replicate r into the host view
-// (large pageable columns are waited for, the rest is not)
+// (columns that landed are copied on, the rest is not waited for)
 int copy_out(ppc_state* s, int32_t r, ppc_agents* a, int32_t first, int32_t n)
 {
 	const int32_t base = s->reps[r].base;
 	const int D = s->ndefs;
 	view& v = s->v;
+	s->landing = s->bounce && (size_t)(n - first) * sizeof(double) >= kBounceLeast && vectors_page_locked(a);
 	PPC_TRY(get_vec(s, a->positions, v.pos[s->cur], r, first, n));
 	PPC_TRY(get_vec(s, a->velocities, v.vel, r, first, n));
 	PPC_TRY(get_vec(s, a->previous_velocities, v.vprev, r, first, n));
@@ -699,12 +703,11 @@ int copy_out(ppc_state* s, int32_t r, ppc_agents* a, int32_t first, int32_t n)
 	PPC_TRY(get_scalar(s, a->agent_ids, v.ids, base, first, n, 1));
 	// the vectors' copies last, so that the host copies of the columns that
 	// landed before them run beside these
-	const uint64_t pieces = s->bounce_pieces;
-	const bool landing = !s->pending_host.empty();
-	if (landing)
+	const bool landed = !s->pending_host.empty();
+	if (landed)
 		PPC_CUDA(cudaEventRecord(s->ev_landed, s->stream));
 	PPC_TRY(flush_copies(s));
-	if (landing && s->bounce_pieces == pieces) // page-locked vectors: none of them uses the landing area
+	if (landed)
 	{
 		PPC_CUDA(cudaEventSynchronize(s->ev_landed));
 		drain_host(s);
@@ -731,7 +734,6 @@ int transfer_out_on(ppc_state* s, int32_t r, ppc_agents* a, cudaStream_t main, b
 	PPC_TRY(rc);
 	PPC_TRY(launch_pull(s));
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
-	drain_host(s);
 	if (beside && *s->pinned_err)
 	{
 		// the rebuild beside the copies may still set error bits: read the
@@ -752,11 +754,11 @@ int transfer_out_on(ppc_state* s, int32_t r, ppc_agents* a, cudaStream_t main, b
 		PPC_TRY(copy_out(s, r, a, guess, n));
 	const int32_t base = s->reps[r].base;
 	view& v = s->v;
+	s->landing = false;
 	if (a->spring_counts)
 	{
 		PPC_TRY(get_scalar(s, a->spring_counts, v.scnt, base, 0, n, 1));
 		PPC_CUDA(cudaStreamSynchronize(s->stream));
-		drain_host(s);
 		int32_t mx = 0;
 		for (int32_t i = 0; i < n; i++)
 			mx = std::max(mx, a->spring_counts[i]);
@@ -772,10 +774,7 @@ int transfer_out_on(ppc_state* s, int32_t r, ppc_agents* a, cudaStream_t main, b
 		}
 	}
 	if (n > guess || a->spring_counts)
-	{
 		PPC_CUDA(cudaStreamSynchronize(s->stream));
-		drain_host(s);
-	}
 	return PPC_OK;
 }
 
@@ -1920,8 +1919,7 @@ int ensure_mot_store(ppc_state* s, int32_t S)
 // rows [base, base + n) of the columns from (to_device) or to the host rows
 int move_columns(ppc_state* s, const std::vector<column>& cols, int32_t base, int32_t n, bool to_device)
 {
-	s->pending_host.clear();
-	s->bounce_used = 0;
+	s->landing = false;
 	for (const auto& c : cols)
 	{
 		if (!c.host || c.width == 0 || n == 0)
@@ -1934,7 +1932,6 @@ int move_columns(ppc_state* s, const std::vector<column>& cols, int32_t base, in
 			PPC_TRY(copy_down(s, const_cast<void*>(c.host), dev, bytes));
 	}
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
-	drain_host(s);
 	return PPC_OK;
 }
 

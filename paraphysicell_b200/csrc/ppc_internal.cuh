@@ -357,13 +357,13 @@ struct ppc_state
 	size_t stage_used = 0; // bytes of the arena taken by the current transfer call
 	std::vector<ppc::pending_unpack> pending_unpacks;
 	std::vector<ppc::pending_copy> pending_copies;
-	// large copies to pageable host rows: their page-locked landing area and
-	// the host copies due once they have landed
+	// large pageable columns of a download with page-locked vectors: their
+	// page-locked landing area and the host copies due once they have landed
 	void* bounce = nullptr;
 	size_t bounce_bytes = 0, bounce_used = 0;
+	bool landing = false; // for the copies being queued
 	ppc::pull_list pull; // jobs of the small download being queued
 	bool pulling = false;
-	uint64_t bounce_pieces = 0; // copies into it so far
 	std::vector<ppc::pending_copy> pending_host;
 
 	// captured CUDA graphs of blocks of fused steps (ppc_api.cu: replay_steps)

@@ -155,3 +155,29 @@ def test_large_downloads_into_pageable_rows(n):
     d.download(third)
     gu.assert_same_state(again, third)
     d.close()
+
+
+@pytest.mark.parametrize("n", [131071, 131072, 300001])
+def test_large_downloads_beside_page_locked_vectors(n):
+    """Pageable columns land beside page-locked vectors until the landing area
+    is full, the rest takes the driver's copies."""
+    from paraphysicell_b200.device import PinnedPool
+
+    mesh, params, a = wl.scaled(wl.config5, n, seed=3, capacity=n + 64)
+    d = Simulation(mesh, params, a.capacity)
+    d.upload(a)
+    pool = PinnedPool()
+    got = AgentArrays(0, a.dims, a.ndefs, a.capacity)
+    for f in ("positions", "orientation"):
+        got.arrays[f] = pool(got.arrays[f].size, np.float64)
+    for _ in range(2):
+        got.count = got.capacity
+        d.download(got, fields=("positions", "orientation", "radius", "total_volume", "agent_ids",
+                                "cell_adhesion_affinities", "flags"))
+        assert got.count == n
+        for f in ("positions", "orientation", "radius", "total_volume", "agent_ids", "cell_adhesion_affinities",
+                  "flags"):
+            assert np.array_equal(got[f], a[f]), f
+            got.arrays[f][:] = 0
+    d.close()
+    pool.free()
