@@ -649,7 +649,6 @@ int transfer_in(ppc_state* s, int32_t r, const ppc_agents* a, bool defaults)
 		return PPC_OK;
 	}
 	invalidate_bins(s);
-	*s->pinned_skin = 1.f; // the fields that decide the skin may have changed
 	// slots were rewritten: the next rebuild counts by slot
 	PPC_CUDA(cudaMemsetAsync(v.order_valid, 0, sizeof(int32_t), s->stream));
 	PPC_CUDA(cudaStreamSynchronize(s->stream));
@@ -954,12 +953,13 @@ int replay_steps(ppc_state* s, int k, bool phenotype, double p_divide, double p_
 static_assert(sizeof(rep_counters) >= 4 * sizeof(int32_t), "the error word and three spare words end the counters");
 
 constexpr int kListLeast = 4;	   // steps of a call that run over lists
+constexpr int kListHold = 32;	   // calls at most between two attempts
+constexpr float kSkinUnknown = 1e30f;
 constexpr int kListSteps = 100000; // steps of one launch over lists
 
 // Whether a call's steps run over neighbour lists: the default launch shape
 // (an explicit other one asks for its own pass), and a mesh that leaves a
-// skin beyond the largest reach (by the uploaded fields; the device reports
-// the skin it found where radii changed there). The launch itself costs about
+// skin beyond the largest reach (by the uploaded fields). The launch itself costs about
 // 13 us over its steps and making lists about as much as one scanning step,
 // so calls of a few steps keep the scanning passes: on 88,700 agents one step
 // after an upload takes 35 us over lists and 28 us scanning, four take about
@@ -967,8 +967,6 @@ constexpr int kListSteps = 100000; // steps of one launch over lists
 bool use_lists(ppc_state* s, int32_t steps)
 {
 	if (!s->lists_fit || !s->queue || s->persistent || s->profiling || steps < kListLeast)
-		return false;
-	if (*static_cast<volatile float*>(s->pinned_skin) <= 0.f)
 		return false;
 	double voxel = 1e30;
 	for (const auto& R : s->reps)
@@ -979,7 +977,24 @@ bool use_lists(ppc_state* s, int32_t steps)
 			return false;
 	// a stream under capture is left to the replayed steps, which refuse it
 	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-	return cudaStreamIsCapturing(s->stream, &cs) == cudaSuccess && cs == cudaStreamCaptureStatusNone;
+	if (cudaStreamIsCapturing(s->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
+		return false;
+	// Lists that the device gave up (they did not fit, had no skin or did not
+	// pay) are tried again after one call, then two, four and so on: a call that
+	// gives them up costs about three rebuilds, and its remaining steps a fifth
+	// more than the scanning passes'.
+	volatile float* skin = s->pinned_skin;
+	if (*skin == 0.f)
+	{
+		s->list_hold = s->list_wait = std::min(kListHold, std::max(1, 2 * s->list_wait));
+		*skin = kSkinUnknown;
+	}
+	else if (*skin < kSkinUnknown)
+		s->list_wait = 0;
+	if (s->list_hold == 0)
+		return true;
+	s->list_hold--;
+	return false;
 }
 
 int run_list_steps(ppc_state* s, int32_t steps)
@@ -1301,7 +1316,7 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 	a.want(v.safff, C * s->ndefs);
 	a.want(v.saff, C * s->ndefs);
 	a.want(v.ncnt, C);
-	a.want(v.lctl, 8);
+	a.want(v.lctl, 16);
 	s->reach_radius.assign(replicates, kRadius);
 	s->reach_factor.assign(replicates, 1.25);
 	a.want(v.bad, C);
@@ -1354,7 +1369,7 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 		}
 		s->pinned_err = reinterpret_cast<int32_t*>(s->pinned_ctr + replicates);
 		s->pinned_skin = reinterpret_cast<float*>(s->pinned_ctr + replicates + 1);
-		*s->pinned_skin = 1.f;
+		*s->pinned_skin = kSkinUnknown;
 	}
 	if (rc == PPC_OK)
 	{

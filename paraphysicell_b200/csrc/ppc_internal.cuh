@@ -227,7 +227,9 @@ enum : int
 	LCTL_WANT = 3,	// the same for the next lists: lowered where a pool of entries was too small
 	LCTL_BUILT = 4, // bits of the skin of the lists in use
 	LCTL_FIT = 5,	// every warp has its lists
-	LCTL_LEFT = 6	// steps a launch over lists left to k_list_rest behind it
+	LCTL_LEFT = 6,	// steps a launch over lists left to k_list_rest behind it
+	LCTL_AGE = 7,	// steps made over the lists in use
+	LCTL_DEBT = 8	// steps by which the lists fell short of paying for themselves
 };
 
 constexpr int32_t kMoved = -2; // view::move_src: the slot's fields changed since the last rebuild
@@ -346,7 +348,9 @@ struct ppc_state
 	bool list_ready[2] = {};	  // the list kernel's shared-memory limit is set (per precision)
 	int rest_blocks[2] = {};	  // blocks of the launch for steps that the lists leave (per precision)
 	std::vector<double> reach_radius, reach_factor; // per replicate: largest uploaded radius and rmad
-	float* pinned_skin = nullptr; // skin of the lists in use, written by the device (0: none)
+	float* pinned_skin = nullptr; // skin of the lists in use, written by the device (0: they were given up)
+	int list_hold = 0;			  // calls that scan the mesh before lists are tried again...
+	int list_wait = 0;			  // ...and how many did last time
 	int64_t launches = 0;
 	int max_grid_blocks = 0;
 	int sm_count = 148;

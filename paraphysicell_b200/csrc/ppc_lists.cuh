@@ -42,7 +42,15 @@ constexpr int kListHits = 12;	  // accepted neighbours a lane orders in shared m
 constexpr int kListFew = 256;	  // block size up to which a thread has registers to spare
 constexpr int kListMost = 255;	  // entries of one list
 constexpr float kSkinMax = 5.0f;  // um; the lists of the default cell radius then hold about twice its neighbours
-constexpr float kSkinMin = 0.5f;  // below it the mesh is rebuilt every step
+constexpr float kSkinMin = 0.5f;  // below it there are no lists
+// Where agents move fast, the lists are soon past their skin. Mesh and lists made
+// anew by the grid cost about as much as five steps over lists save against
+// scanning (2,000 to 80,000 agents: 86 to 145 us against 16 to 24 us a step), so
+// each rebuild adds five steps less those its lists lasted to a debt, and a call
+// whose debt is past the limit goes on without lists. The limit admits the
+// first steps of a relaxing tissue (96 replicates placed at random: lists that
+// last 1, 4, 7, 11, 17 steps) and stops at the third list that lasts one step.
+constexpr int kListPays = 5, kListDebt = 8;
 constexpr int32_t kStill = 1 << 30; // list entries: the neighbour is not movable
 
 // events in the upper half of a barrier word
@@ -364,9 +372,13 @@ __global__ void __launch_bounds__(kThreads) k_list_prepare(view v, int reset)
 	if (t == 0)
 	{
 		if (reset)
+		{
 			v.lctl[LCTL_WANT] = __float_as_int(kSkinMax);
+			v.lctl[LCTL_DEBT] = 0;
+		}
 		v.lctl[LCTL_CAP] = v.lctl[LCTL_WANT];
 		v.lctl[LCTL_FIT] = 1;
+		v.lctl[LCTL_AGE] = 0;
 		*v.nl_used = 0;
 	}
 	list_reach(v, t < n ? v.spos4[t].w : 0.0);
@@ -1080,12 +1092,12 @@ __device__ __forceinline__ unsigned long long list_wait(const view& v, const lis
 	return b.out;
 }
 
-// Container update (after a removal), mesh and lists rebuilt by the whole
-// grid; the new key-ordered rows go to lpos[p]. `flushed`: the slot-ordered
-// rows are current. Returns false when a barrier gave up.
+// Container update (after a removal), mesh and (`lists`) lists rebuilt by the
+// whole grid; the new key-ordered rows go to lpos[p]. `flushed`: the
+// slot-ordered rows are current. Returns false when a barrier gave up.
 template <int DIMS>
 __device__ __forceinline__ bool list_rebuild(const view& v, const list_args& a, list_barrier& bar, int p, bool remove,
-										  bool flushed, unsigned char* smem)
+										  bool flushed, bool lists, unsigned char* smem)
 {
 	const int T = blockDim.x, t0 = blockIdx.x * T + threadIdx.x, step = gridDim.x * T;
 	const int cur = a.cur;
@@ -1115,7 +1127,7 @@ __device__ __forceinline__ bool list_rebuild(const view& v, const list_args& a, 
 			v.lctl[LCTL_REACH] = 0;
 			v.lctl[LCTL_DIRTY] = 0;
 			v.lctl[LCTL_CAP] = v.lctl[LCTL_WANT];
-			v.lctl[LCTL_FIT] = 1;
+			v.lctl[LCTL_FIT] = lists ? 1 : 0;
 			*v.nl_used = 0;
 		}
 		for (int t = blockIdx.x * T; t < v.total_cap; t += step)
@@ -1137,12 +1149,14 @@ __device__ __forceinline__ bool list_rebuild(const view& v, const list_args& a, 
 		bin_finish(v, t0, step);
 		if (list_wait(v, a, bar, 0) == ~0ull)
 			return false;
-		const float skin = list_skin(v, a.voxel);
+		const float skin = lists ? list_skin(v, a.voxel) : 0.0f;
 		if (blockIdx.x == 0 && threadIdx.x == 0)
 		{
 			*a.skin_out = skin;
 			v.lctl[LCTL_BUILT] = __float_as_int(skin);
 		}
+		if (!lists)
+			return list_wait(v, a, bar, 0) != ~0ull;
 		list_warp& w = reinterpret_cast<list_warp*>(smem)[threadIdx.x >> 5];
 		for (int tb = blockIdx.x * T; tb < n; tb += step)
 			list_build<DIMS, 2>(v, cur, p, tb + (threadIdx.x & ~31), n, skin, a.opts & FUSED_SPRINGS, w);
@@ -1158,8 +1172,9 @@ __device__ __forceinline__ bool list_rebuild(const view& v, const list_args& a, 
 // The steps of a call. RESIDENT: the grid has a thread for every agent, which
 // keeps the agent's rows and the first entries of its list in shared memory
 // between the steps. The launch runs while every warp has its lists; where
-// some do not fit, or no skin is left, it leaves the rest of the call
-// (LCTL_LEFT), with the mesh current, to k_list_rest behind it.
+// some do not fit, no skin is left, or they do not pay (kListDebt), it leaves
+// the rest of the call (LCTL_LEFT), with the mesh current, to k_list_rest
+// behind it.
 template <int DIMS, bool F32, bool RESIDENT, int MOST>
 __global__ void __launch_bounds__(MOST, 1)
 	k_list_steps(const __grid_constant__ view v, const __grid_constant__ list_args a)
@@ -1191,7 +1206,9 @@ __global__ void __launch_bounds__(MOST, 1)
 	int n = *v.cursor;
 	int p = a.p;
 	float skin = lctl_float(v, LCTL_BUILT);
-	bool rebuild = v.lctl[LCTL_DIRTY] != 0 || lctl_float(v, LCTL_WANT) < skin;
+	bool past = v.lctl[LCTL_DIRTY] != 0;
+	const bool cut = lctl_float(v, LCTL_WANT) < skin; // lists that did not fit
+	int age = v.lctl[LCTL_AGE], debt = v.lctl[LCTL_DEBT];
 	if (a.refresh)
 	{
 		unsigned long long ev = 0;
@@ -1200,8 +1217,16 @@ __global__ void __launch_bounds__(MOST, 1)
 		ev = list_wait(v, a, bar, ev);
 		if (ev == ~0ull)
 			return;
-		rebuild = rebuild || ev != 0;
+		past = past || ev != 0;
 	}
+	bool rebuild = past || cut, lists = true;
+	auto charge = [&]() { // lists that lasted `age` steps are to be made anew
+		debt = max(0, debt + kListPays - age);
+		age = 0;
+		lists = debt <= kListDebt;
+	};
+	if (past)
+		charge();
 	// past this barrier no block reads the control words of the old lists
 	if (rebuild && list_wait(v, a, bar, 0) == ~0ull)
 		return;
@@ -1226,7 +1251,7 @@ __global__ void __launch_bounds__(MOST, 1)
 	{
 		if (rebuild)
 		{
-			if (!list_rebuild<DIMS>(v, a, bar, p, replay, flushed, smem))
+			if (!list_rebuild<DIMS>(v, a, bar, p, replay, flushed, lists, smem))
 				return;
 			n = *v.cursor;
 			skin = lctl_float(v, LCTL_BUILT);
@@ -1256,15 +1281,19 @@ __global__ void __launch_bounds__(MOST, 1)
 				ev |= list_step<DIMS, F32, BATCH>(v, a, reps, lc, w, own, p, t, n, k == 0, last, skin);
 			}
 		p ^= 1;
+		age++;
 		ev = list_wait(v, a, bar, ev);
 		if (ev == ~0ull)
 			return;
 		rebuild = false;
 		if (ev == 0)
 			continue;
-		const bool remove = ev >= kEventRemove, past = (unsigned)(ev >> 32 & 0xffff) != 0;
+		const bool remove = ev >= kEventRemove;
+		past = (unsigned)(ev >> 32 & 0xffff) != 0;
 		replay = remove && a.springs;
 		rebuild = replay || (past && !last);
+		if (rebuild)
+			charge();
 		flushed = last;
 		if (past && last && !replay && t0 == 0)
 			v.lctl[LCTL_DIRTY] = 1; // the next call rebuilds first
@@ -1277,6 +1306,11 @@ __global__ void __launch_bounds__(MOST, 1)
 			if (RESIDENT && !rebuild && !last)
 				reload();
 		}
+	}
+	if (t0 == 0)
+	{
+		v.lctl[LCTL_AGE] = age;
+		v.lctl[LCTL_DEBT] = debt;
 	}
 	if (blockIdx.x == 0 && v.auto_springs)
 		for (int r = threadIdx.x; r < v.nreps; r += T)
@@ -1345,7 +1379,11 @@ __global__ void __launch_bounds__(kPersistThreads)
 		for (int t = t0 + threadIdx.x; t < v.total_cap; t += step)
 			v.pos[a.cur][t] = v.pos[cur][t];
 	if (blockIdx.x == 0 && threadIdx.x == 0)
+	{
 		v.lctl[LCTL_DIRTY] = 1;
+		v.lctl[LCTL_AGE] = kListPays; // the rebuild that the next lists start from is not theirs
+		v.lctl[LCTL_DEBT] = 0;
+	}
 	if (blockIdx.x == 0 && v.auto_springs)
 		for (int r = threadIdx.x; r < v.nreps; r += T)
 			v.ctr[r].spring_epoch += a.steps;

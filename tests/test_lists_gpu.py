@@ -177,6 +177,34 @@ def test_two_live_states_of_different_capacity(capacities):
 
 
 @pytest.mark.parametrize("form", FORMS)
+def test_agents_too_fast_for_lists(form):
+    """Repulsion that throws agents past the skin at every step: the call goes
+    on without lists, and the calls after it scan the mesh (many launches
+    instead of a few), until calmer tissue gets lists again."""
+    mesh, params, a = _agents(700, 3, 130, 61, FORMS[form])
+    params.virtual_wall_at_domain_edges = 1
+    a.arrays["cell_cell_repulsion_strength"][: a.count] = 2000.0
+    o, d = make_pair(mesh, params, a)
+
+    def call(k):
+        before = d.launches()
+        _run(o, d, a, (k,))
+        return d.launches() - before
+
+    assert call(12) < 24  # lists, as far as they go
+    assert call(9) > 36
+    h = fetch(d, a)
+    h.arrays["cell_cell_repulsion_strength"][: h.count] = 1e-3
+    h.arrays["cell_cell_adhesion_strength"][: h.count] = 1e-3
+    h.arrays["previous_velocities"][: 3 * h.count] = 0.0
+    h.arrays["positions"][: 3 * h.count] = np.random.default_rng(1).uniform(-120, 120, 3 * h.count)
+    o.upload(h)
+    d.upload(h)
+    assert min(call(20) for _ in range(4)) < 40
+    d.close()
+
+
+@pytest.mark.parametrize("form", FORMS)
 def test_barrier_timeout_is_reported_and_recoverable(form):
     """A one-poll wait limit makes the grid barriers of a call over lists give
     up: PPC_ERR_TIMEOUT at the next synchronising call, steps refused until the
