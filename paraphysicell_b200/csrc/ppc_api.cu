@@ -950,6 +950,37 @@ int replay_steps(ppc_state* s, int k, bool phenotype, double p_divide, double p_
 	return PPC_OK;
 }
 
+// The lists' arrays, about 1.1 KB per slot, made by the first call that uses
+// them: a state that steps once a call, or divides, never does. A device
+// without room for them runs every step through the scanning passes.
+bool lists_allocated(ppc_state* s)
+{
+	if (s->lists_tried)
+		return s->lists_fit;
+	s->lists_tried = true;
+	const size_t C = s->total_cap;
+	view& v = s->v;
+	v.nl_pool = 24 * (int64_t)C + 8192;
+	arena a;
+	a.want(v.nl_used, 1);
+	a.want(s->list_bar, 64);
+	a.want(v.lpos[0], C, false);
+	a.want(v.lpos[1], C, false);
+	a.want(v.lvprev, C, false);
+	a.want(v.lpress, C, false);
+	a.want(v.nlc, C, false);
+	a.want(v.nl_slab, C / 32 + 1, false);
+	a.want(v.nl, v.nl_pool, false);
+	a.want(v.nl_pair, v.nl_pool, false);
+	a.want(v.lspr, C * s->scap, false);
+	a.want(v.lcoef, C * s->scap, false);
+	a.want(v.tpos, C, false);
+	s->lists_fit = a.place(s) == PPC_OK;
+	if (!s->lists_fit)
+		cudaGetLastError(); // no room is not an error of the state
+	return s->lists_fit;
+}
+
 static_assert(sizeof(rep_counters) >= 4 * sizeof(int32_t), "the error word and three spare words end the counters");
 
 constexpr int kListLeast = 4;	   // steps of a call that run over lists
@@ -966,7 +997,7 @@ constexpr int kListSteps = 100000; // steps of one launch over lists
 // the same, sixty 0.67 ms and 1.9 ms.
 bool use_lists(ppc_state* s, int32_t steps)
 {
-	if (!s->lists_fit || !s->queue || s->persistent || s->profiling || steps < kListLeast)
+	if ((s->lists_tried && !s->lists_fit) || !s->queue || s->persistent || s->profiling || steps < kListLeast)
 		return false;
 	double voxel = 1e30;
 	for (const auto& R : s->reps)
@@ -992,7 +1023,7 @@ bool use_lists(ppc_state* s, int32_t steps)
 	else if (*skin < kSkinUnknown)
 		s->list_wait = 0;
 	if (s->list_hold == 0)
-		return true;
+		return lists_allocated(s);
 	s->list_hold--;
 	return false;
 }
@@ -1083,32 +1114,6 @@ int run_steps(ppc_state* s, int32_t steps, bool phenotype, double p_divide, doub
 	}
 	s->lists_stale = steps > 0 || s->lists_stale;
 	return mark_ready(s);
-}
-
-// The lists' arrays, about 1.4 KB per agent. A device without room for them
-// beside the state runs every step through the scanning passes.
-void alloc_lists(ppc_state* s)
-{
-	const size_t C = s->total_cap;
-	view& v = s->v;
-	v.nl_pool = 24 * (int64_t)C + 8192;
-	arena a;
-	a.want(v.nl_used, 1);
-	a.want(s->list_bar, 64);
-	a.want(v.lpos[0], C, false);
-	a.want(v.lpos[1], C, false);
-	a.want(v.lvprev, C, false);
-	a.want(v.lpress, C, false);
-	a.want(v.nlc, C, false);
-	a.want(v.nl_slab, C / 32 + 1, false);
-	a.want(v.nl, v.nl_pool, false);
-	a.want(v.nl_pair, v.nl_pool, false);
-	a.want(v.lspr, C * s->scap, false);
-	a.want(v.lcoef, C * s->scap, false);
-	a.want(v.tpos, C, false);
-	s->lists_fit = a.place(s) == PPC_OK;
-	if (!s->lists_fit)
-		cudaGetLastError(); // no room is not an error of the state
 }
 
 // grid of a mesh (validated: positive voxel shapes, maxs >= mins); sizes in
@@ -1346,8 +1351,6 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 		rc = fail(PPC_ERR_CUDA, "cudaMemset failed");
 	if (rc == PPC_OK && cudaMemsetAsync(v.move_src, 0xff, sizeof(int32_t) * std::max<size_t>(C, 1), s->stream) != cudaSuccess)
 		rc = fail(PPC_ERR_CUDA, "cudaMemset failed");
-	if (rc == PPC_OK)
-		alloc_lists(s);
 	s->host_count.assign(replicates, 0);
 	if (rc == PPC_OK
 		&& cudaHostAlloc(reinterpret_cast<void**>(&s->pinned_ctr), sizeof(rep_counters) * (replicates + 2),

@@ -341,7 +341,8 @@ struct ppc_state
 	bool skin_lists = false;
 	bool skin_refresh = false;
 	bool skin_reset = true;		  // a full upload since lists were made
-	bool lists_fit = false;		  // the device had room for the lists
+	bool lists_tried = false;	  // the lists' arrays were asked for...
+	bool lists_fit = false;		  // ...and the device had room for them
 	int lcur = 0;				  // lpos buffer that holds the positions
 	int bar_set = 0;			  // barrier words of the next list launch
 	unsigned long long* list_bar = nullptr; // [2 sets * 2 words * 16]

@@ -5,6 +5,7 @@ one thread per agent in small or large blocks, or several agents per thread."""
 import numpy as np
 import pytest
 
+from paraphysicell_b200 import build
 from paraphysicell_b200 import workloads as wl
 from paraphysicell_b200.abi import PPC_ERR_ARG, PPC_ERR_TIMEOUT, AgentArrays, Mesh, Params, PPCError
 
@@ -223,6 +224,31 @@ def test_barrier_timeout_is_reported_and_recoverable(form):
     d.set_wait_limit(1 << 25)
     d.upload(a)
     _run(o, d, a, (5, 12, 1, 9))
+    d.close()
+
+
+def test_only_calls_over_lists_take_their_memory():
+    """200,000 slots: the lists' arrays (some 220 MB) come with the first call
+    that steps over lists, not with the state, its uploads or single steps."""
+    import torch
+
+    from paraphysicell_b200.device import Simulation
+
+    mesh, params, a = _agents(2000, 3, 150, 71, 200000)
+    build.ensure_built()
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    d = Simulation(mesh, params, a.capacity)
+    d.upload(a)
+    for _ in range(3):
+        d.step(1)
+    d.step_with_phenotype(5, 0.0, 0.0)
+    fetch(d, a)
+    taken = free - torch.cuda.mem_get_info()[0]
+    assert taken < 300 << 20
+    d.step(8)
+    d.synchronize()
+    assert free - torch.cuda.mem_get_info()[0] > taken + (100 << 20)
     d.close()
 
 
