@@ -193,7 +193,9 @@ int ppc_set_random_seed(ppc_state* s, uint64_t seed);
  *     shared memory (32 KiB is a good budget; a block whose ranges do not fit
  *     reads global memory).
  * `threads` per block 32..256, a multiple of 32 (the fused pass uses at most
- * 128). Results do not depend on the shape; ppc_autotune picks one. */
+ * 128). Results do not depend on the shape; ppc_autotune picks one. Calls of
+ * several steps over neighbour lists (ppc_step) have no such shape: a shape
+ * other than -4 set here asks for its pass and runs every step with it. */
 int ppc_set_launch_shape(ppc_state* s, int32_t tile_edge, int32_t threads, int32_t smem_bytes);
 
 /* How ppc_step runs a mechanics step (ppc_step_with_phenotype and steps with
@@ -220,9 +222,10 @@ int ppc_set_wait_limit(ppc_state* s, int64_t polls);
  * OpenMP loops have no launch shape): runs 2 x `steps` mechanics steps
  * (ppc_step) with each candidate shape — -4, -3, -1 and -2 with 128 threads,
  * 0 with 128 threads / 32 KiB and with 64 threads / 16 KiB — times the second
- * half of each on the state's stream, and keeps the fastest. The simulation
- * advances by 12 x `steps` steps (the trajectory does not depend on the
- * shape). Writes the chosen shape to `tile_edge` and `threads` when they are
+ * half of each on the state's stream, and keeps the fastest for the calls
+ * that run the fused pass; calls over neighbour lists (ppc_step) stay on. The
+ * simulation advances by 12 x `steps` steps (the trajectory does not depend on
+ * the shape). Writes the chosen shape to `tile_edge` and `threads` when they are
  * not NULL. */
 int ppc_autotune(ppc_state* s, int32_t steps, int32_t* tile_edge, int32_t* threads);
 
@@ -515,8 +518,12 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t replicate, ppc_inter
 
 /* ---- fused step ----------------------------------------------------------- */
 /* ppc_step returns once the work is queued (device errors surface at the
- * next ppc_synchronize or syncing call). Blocks of steps are captured once in
- * a CUDA graph and replayed. */
+ * next ppc_synchronize or syncing call). Calls of four steps and more run in
+ * one launch over neighbour lists that outlive a step, while agents move little
+ * enough and the mesh's voxels leave room beside the largest interaction
+ * reach; the first such call of a state allocates the lists, about 1.1 KB a
+ * slot. All other steps scan the mesh; blocks of them are captured once in a
+ * CUDA graph and replayed. Both give the same results. */
 
 /* Advances `steps` mechanics steps in the order of simulator::simulate_mechanics
  * (reference: src/simulator.cpp:157-196, without gradient, custom rules,

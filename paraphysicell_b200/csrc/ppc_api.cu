@@ -988,8 +988,8 @@ constexpr int kListHold = 32;	   // calls at most between two attempts
 constexpr float kSkinUnknown = 1e30f;
 constexpr int kListSteps = 100000; // steps of one launch over lists
 
-// Whether a call's steps run over neighbour lists: the default launch shape
-// (an explicit other one asks for its own pass), and a mesh that leaves a
+// Whether a call's steps run over neighbour lists: the default launch shape or
+// the autotuner's (a caller's choice of another one asks for its own pass), and a mesh that leaves a
 // skin beyond the largest reach (by the uploaded fields). The launch itself costs about
 // 13 us over its steps and making lists about as much as one scanning step,
 // so calls of a few steps keep the scanning passes: on 88,700 agents one step
@@ -997,7 +997,7 @@ constexpr int kListSteps = 100000; // steps of one launch over lists
 // the same, sixty 0.67 ms and 1.9 ms.
 bool use_lists(ppc_state* s, int32_t steps)
 {
-	if ((s->lists_tried && !s->lists_fit) || !s->queue || s->persistent || s->profiling || steps < kListLeast)
+	if ((s->lists_tried && !s->lists_fit) || s->scan_only || s->persistent || s->profiling || steps < kListLeast)
 		return false;
 	double voxel = 1e30;
 	for (const auto& R : s->reps)
@@ -1484,6 +1484,7 @@ int ppc_set_launch_shape(ppc_state* s, int32_t tile_edge, int32_t threads, int32
 	release_graph(s);
 	s->flat = tile_edge == -3;
 	s->queue = tile_edge == -4;
+	s->scan_only = !s->queue; // a caller's own choice; ppc_autotune's leaves the lists on
 	s->staged = tile_edge == 0;
 	s->coop = tile_edge == 0 || tile_edge == -2;
 	s->tile_threads = threads;
@@ -2297,6 +2298,7 @@ int ppc_autotune(ppc_state* s, int32_t steps, int32_t* tile_edge, int32_t* threa
 	for (int k = 0; k < ncand && rc == PPC_OK; k++)
 	{
 		rc = ppc_set_launch_shape(s, cand[k].edge, cand[k].threads, cand[k].smem);
+		s->scan_only = true; // the shapes' own passes are compared
 		if (rc == PPC_OK)
 			rc = run_steps(s, steps, false, 0, 0); // warm-up: graph capture of this shape
 		if (rc != PPC_OK)
@@ -2318,8 +2320,10 @@ int ppc_autotune(ppc_state* s, int32_t steps, int32_t* tile_edge, int32_t* threa
 	}
 	cudaEventDestroy(e0);
 	cudaEventDestroy(e1);
+	s->scan_only = false;
 	PPC_TRY(rc);
 	PPC_TRY(ppc_set_launch_shape(s, cand[best].edge, cand[best].threads, cand[best].smem));
+	s->scan_only = false;
 	if (tile_edge)
 		*tile_edge = cand[best].edge;
 	if (threads)

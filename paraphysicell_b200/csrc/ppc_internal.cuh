@@ -399,6 +399,7 @@ struct ppc_state
 	bool coop = false;
 	bool flat = false; // per-thread pass with batched candidate fetches (shape -3)
 	bool queue = true; // per-thread pass with the warp's candidates shared out (shape -4, the default)
+	bool scan_only = false; // every step runs the fused pass: its launch shape was chosen by the caller
 	bool produce = false; // the fused pass being launched makes the rebuild's entries (FUSED_PRODUCE)
 	bool persistent = false;		 // mechanics steps as one cooperative launch each (PPC_STEP_PERSISTENT)
 	long long wait_limit = 1LL << 25; // polls of a bounded device wait before it gives up

@@ -227,6 +227,32 @@ def test_barrier_timeout_is_reported_and_recoverable(form):
     d.close()
 
 
+@pytest.mark.parametrize("shrink", [0.8, 1.0])
+@pytest.mark.parametrize("steps", [2, 3, 10])
+def test_autotuned_states_step_over_lists(steps, shrink):
+    """Whatever shape wins for the fused pass (-2 where agents are dense), long
+    calls run over lists; a shape the caller sets runs every step."""
+    mesh, params, a = wl.config2(seed=2)
+    a.arrays["positions"][:] *= shrink
+    _, d = make_pair(mesh, params, a)
+    d.update_mechanics_mesh()
+    d.step(100)  # past the tissue's first relaxation
+    d.autotune(steps)
+
+    def launches():
+        before = d.launches()
+        d.step(60)
+        d.synchronize()
+        return d.launches() - before
+
+    assert launches() < 20
+    d.set_launch_shape(-3, 128, 0)
+    assert launches() >= 240
+    d.set_launch_shape(-4, 128, 0)
+    assert launches() < 20
+    d.close()
+
+
 def test_only_calls_over_lists_take_their_memory():
     """200,000 slots: the lists' arrays (some 220 MB) come with the first call
     that steps over lists, not with the state, its uploads or single steps."""
