@@ -297,7 +297,9 @@ struct graph_entry
 struct ppc_state
 {
 	int device = 0;
-	int32_t dims = 3, ndefs = 1, nreps = 1, total_cap = 0, scap = 12, ncap = 64;
+	static constexpr int32_t scap = 12; // springs per agent
+	static_assert(scap <= 64, "k_spring_detach holds a row's positions in the bits of a word");
+	int32_t dims = 3, ndefs = 1, nreps = 1, total_cap = 0, ncap = 64;
 	ppc_params params {};
 	std::vector<ppc_mesh> meshes;
 	std::vector<ppc::rep_info> reps;

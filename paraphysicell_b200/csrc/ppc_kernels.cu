@@ -3159,116 +3159,53 @@ __global__ void k_spring_detach(view v)
 	const int base = v.reps[r].base;
 	const uint64_t ep = (uint64_t)v.ctr[r].spring_epoch;
 	const int32_t* row = v.springs + (int64_t)s * v.scap;
-	if (v.scap <= 64)
-	{
-		// rows as bit masks of their positions, in registers
-		uint64_t seen = 0, gone = 0;
-		for (int k = 0; k < n; k++)
-		{
-			if ((seen >> k) & 1)
-				continue; // pair handled at its first entry
-			const int j = row[k];
-			const int32_t* rowj = v.springs + (int64_t)j * v.scap;
-			const int nj = v.scnt[j];
-			const double rate_j = v.drate[j], rate_s = v.drate[s];
-			uint64_t P = 0, Q = 0;
-			for (int q = k, c = 0; q < n; q++)
-				if (row[q] == j)
-				{
-					seen |= 1ull << q;
-					if (c++ < kMaxSpringCopies)
-						P |= 1ull << q;
-				}
-			for (int q = 0, c = 0; q < nj; q++)
-				if (rowj[q] == s && c++ < kMaxSpringCopies)
-					Q |= 1ull << q;
-			// a walks first: its entries A name b, b's entries B name a
-			const bool s_first = li < j - base;
-			const int la = s_first ? li : j - base, lb = s_first ? j - base : li;
-			const double ra = (s_first ? rate_s : rate_j) * v.dt, rb = (s_first ? rate_j : rate_s) * v.dt;
-			const uint64_t A = s_first ? P : Q, B = s_first ? Q : P;
-			uint64_t ea = 0, eb = 0; // erased entries
-			for (uint64_t m = A; m; m &= m - 1)
-				if (ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)la, 1024u + (uint64_t)(__ffsll((long long)m) - 1)) <= ra)
-				{
-					ea |= m & (~m + 1);
-					const uint64_t left = B & ~eb;
-					eb |= left & (~left + 1);
-				}
-			for (uint64_t m = B; m; m &= m - 1)
-				if (!(eb & m & (~m + 1))
-					&& ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)lb, 1024u + (uint64_t)(__ffsll((long long)m) - 1)) <= rb)
-				{
-					eb |= m & (~m + 1);
-					const uint64_t left = A & ~ea;
-					ea |= left & (~left + 1);
-				}
-			gone |= s_first ? ea : eb;
-		}
-		for (int k = 0; k < n; k++)
-			v.sdel[(int64_t)s * v.scap + k] = (gone >> k) & 1;
-		v.skeep[s] = n - __popcll(gone);
-		return;
-	}
-	for (int k = 0; k < n; k++)
-		v.sdel[(int64_t)s * v.scap + k] = 0;
+	// rows as bit masks of their positions, in registers
+	uint64_t seen = 0, gone = 0;
 	for (int k = 0; k < n; k++)
 	{
+		if ((seen >> k) & 1)
+			continue; // pair handled at its first entry
 		const int j = row[k];
-		bool seen = false; // pair handled at its first entry
-		for (int q = 0; q < k && !seen; q++)
-			seen = row[q] == j;
-		if (seen)
-			continue;
 		const int32_t* rowj = v.springs + (int64_t)j * v.scap;
 		const int nj = v.scnt[j];
-		int P[kMaxSpringCopies], Q[kMaxSpringCopies];
-		int np = 0, nq = 0;
-		for (int q = k; q < n && np < kMaxSpringCopies; q++)
+		const double rate_j = v.drate[j], rate_s = v.drate[s];
+		uint64_t P = 0, Q = 0;
+		for (int q = k, c = 0; q < n; q++)
 			if (row[q] == j)
-				P[np++] = q;
-		for (int q = 0; q < nj && nq < kMaxSpringCopies; q++)
-			if (rowj[q] == s)
-				Q[nq++] = q;
+			{
+				seen |= 1ull << q;
+				if (c++ < kMaxSpringCopies)
+					P |= 1ull << q;
+			}
+		for (int q = 0, c = 0; q < nj; q++)
+			if (rowj[q] == s && c++ < kMaxSpringCopies)
+				Q |= 1ull << q;
 		// a walks first: its entries A name b, b's entries B name a
 		const bool s_first = li < j - base;
 		const int la = s_first ? li : j - base, lb = s_first ? j - base : li;
-		const double ra = (s_first ? v.drate[s] : v.drate[j]) * v.dt;
-		const double rb = (s_first ? v.drate[j] : v.drate[s]) * v.dt;
-		const int* A = s_first ? P : Q;
-		const int* B = s_first ? Q : P;
-		const int na = s_first ? np : nq, nb = s_first ? nq : np;
-		bool ea[kMaxSpringCopies], eb[kMaxSpringCopies];
-		for (int q = 0; q < kMaxSpringCopies; q++)
-			ea[q] = eb[q] = false;
-		for (int q = 0; q < na; q++)
-			if (ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)la, 1024u + (uint64_t)A[q]) <= ra)
+		const double ra = (s_first ? rate_s : rate_j) * v.dt, rb = (s_first ? rate_j : rate_s) * v.dt;
+		const uint64_t A = s_first ? P : Q, B = s_first ? Q : P;
+		uint64_t ea = 0, eb = 0; // erased entries
+		for (uint64_t m = A; m; m &= m - 1)
+			if (ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)la, 1024u + (uint64_t)(__ffsll((long long)m) - 1)) <= ra)
 			{
-				ea[q] = true;
-				int f = 0;
-				while (f < nb && eb[f])
-					f++;
-				if (f < nb)
-					eb[f] = true;
+				ea |= m & (~m + 1);
+				const uint64_t left = B & ~eb;
+				eb |= left & (~left + 1);
 			}
-		for (int q = 0; q < nb; q++)
-			if (!eb[q] && ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)lb, 1024u + (uint64_t)B[q]) <= rb)
+		for (uint64_t m = B; m; m &= m - 1)
+			if (!(eb & m & (~m + 1))
+				&& ppc_uniform(v.seed, ep, (uint64_t)r, (uint64_t)lb, 1024u + (uint64_t)(__ffsll((long long)m) - 1)) <= rb)
 			{
-				eb[q] = true;
-				int f = 0;
-				while (f < na && ea[f])
-					f++;
-				if (f < na)
-					ea[f] = true;
+				eb |= m & (~m + 1);
+				const uint64_t left = A & ~ea;
+				ea |= left & (~left + 1);
 			}
-		const bool* mine = s_first ? ea : eb;
-		for (int q = 0; q < np; q++)
-			v.sdel[(int64_t)s * v.scap + P[q]] = mine[q] ? 1 : 0;
+		gone |= s_first ? ea : eb;
 	}
-	int kept = 0;
 	for (int k = 0; k < n; k++)
-		kept += v.sdel[(int64_t)s * v.scap + k] == 0;
-	v.skeep[s] = kept;
+		v.sdel[(int64_t)s * v.scap + k] = (gone >> k) & 1;
+	v.skeep[s] = n - __popcll(gone);
 }
 
 __global__ void k_spring_compact_rows(view v)
