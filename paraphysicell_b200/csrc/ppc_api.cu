@@ -182,7 +182,11 @@ void drain_host(ppc_state* s)
 }
 
 // Rows up to this size go between mapped host rows and the device by kernels,
-// which cost less than copies' latency: a download's columns in one launch.
+// which cost less than copies' latency: a download's columns in one launch. A
+// host loop (upload, step, download) of 2,700 agents, at the line: 67 us, 87
+// with copies. Kernels are the faster ones beyond it too (20,000 agents: 105 and
+// 128 us) where nothing else runs; larger rows keep the copies, which run on the
+// transfer stream beside the device's earlier work.
 constexpr size_t kSmallRows = 64 * 1024;
 
 // takes a column of a small download into the launch that follows; false where
@@ -975,7 +979,11 @@ bool lists_allocated(ppc_state* s)
 	a.want(v.lspr, C * s->scap, false);
 	a.want(v.lcoef, C * s->scap, false);
 	a.want(v.tpos, C, false);
+	// a capture on another stream of the program stays valid
+	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+	cudaThreadExchangeStreamCaptureMode(&mode);
 	s->lists_fit = a.place(s) == PPC_OK;
+	cudaThreadExchangeStreamCaptureMode(&mode);
 	if (!s->lists_fit)
 		cudaGetLastError(); // no room is not an error of the state
 	return s->lists_fit;
@@ -990,11 +998,11 @@ constexpr int kListSteps = 100000; // steps of one launch over lists
 
 // Whether a call's steps run over neighbour lists: the default launch shape or
 // the autotuner's (a caller's choice of another one asks for its own pass), and a mesh that leaves a
-// skin beyond the largest reach (by the uploaded fields). The launch itself costs about
-// 13 us over its steps and making lists about as much as one scanning step,
-// so calls of a few steps keep the scanning passes: on 88,700 agents one step
-// after an upload takes 35 us over lists and 28 us scanning, four take about
-// the same, sixty 0.67 ms and 1.9 ms.
+// skin beyond the largest reach (by the uploaded fields). The launch itself
+// costs about 13 us over its steps and making lists about as much as one scanning
+// step, so calls of a few steps keep the scanning passes. 88,700 agents, calls of
+// four steps in a row: 48 us a call over lists, 125 scanning; each followed by a
+// neighbour query, which takes the mesh back: 123 and 159 us.
 bool use_lists(ppc_state* s, int32_t steps)
 {
 	if ((s->lists_tried && !s->lists_fit) || s->scan_only || s->persistent || s->profiling || steps < kListLeast)
@@ -1011,9 +1019,9 @@ bool use_lists(ppc_state* s, int32_t steps)
 	if (cudaStreamIsCapturing(s->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone)
 		return false;
 	// Lists that the device gave up (they did not fit, had no skin or did not
-	// pay) are tried again after one call, then two, four and so on: a call that
-	// gives them up costs about three rebuilds, and its remaining steps a fifth
-	// more than the scanning passes'.
+	// pay) are tried again after one call, then two, four and so on: the call
+	// that gives them up takes longer than scanning would (its first 20 steps:
+	// 14,300 agents 1.52 and 1.42 ms, 80,000 2.51 and 2.24).
 	volatile float* skin = s->pinned_skin;
 	if (*skin == 0.f)
 	{

@@ -28,20 +28,25 @@
 // barrier and a chain of one gather and the FP64 pair code, all latency (so
 // each agent's rows and list stay on chip between the steps); beyond that the
 // latency of the gathers under too few warps, then the bytes of the agents'
-// rows. Measured on one B200, 60 steps and the download of their result,
-// before (mesh rebuilt and searched every step) and now: 900 agents in 2-D
-// 1.00 and 0.30 ms, 14,300 in 3-D 1.99 and 0.60 ms, 88,700 with springs 1.91
-// and 0.67 ms, 96 replicates with 1.03 M agents 55 and 22 ms. Of a step's
+// rows. Measured on one B200, 60 steps and the download of their result, with
+// the mesh rebuilt and searched every step and so: 900 agents in 2-D 1.02 and
+// 0.27 ms, 14,300 in 3-D 1.98 and 0.60 ms, 88,700 with springs 1.92 and 0.67
+// ms, 96 replicates with 1.03 M agents 55 and 22 ms. Of a step's
 // 7,900 cycles for 900 agents the barrier takes 3,300 (of which 2,700 remain
 // with nothing stored before it) and the agents' chain 4,300.
 
-constexpr int kListThreads = 640; // one block per SM: 148 arrivals per barrier; 96 registers a thread
+constexpr int kListThreads = 640; // one block per SM: 148 arrivals per barrier; 96 registers a thread (in 3-D 66
+								  // bytes of them spilled, in 2-D 114)
 constexpr int kListLoop = 512;	  // the same where a thread takes several agents: 128 registers
 constexpr size_t kListSmem = 200 * 1024; // shared bytes of a block, most of them cached list entries
 constexpr int kListHits = 12;	  // accepted neighbours a lane orders in shared memory
 constexpr int kListFew = 256;	  // block size up to which a thread has registers to spare
 constexpr int kListMost = 255;	  // entries of one list
-constexpr float kSkinMax = 5.0f;  // um; the lists of the default cell radius then hold about twice its neighbours
+// um; the lists of the default cell radius then hold about twice its neighbours.
+// 60 steps of 14,300 agents placed at random, and after 120 steps: 1.05 and 0.62
+// ms with 3 um, 0.85 and 0.55 with 5, the same with 8, which the pool of 24
+// entries a slot admits in sparse tissue only.
+constexpr float kSkinMax = 5.0f;
 constexpr float kSkinMin = 0.5f;  // below it there are no lists
 // Where agents move fast, the lists are soon past their skin. Mesh and lists made
 // anew by the grid cost about as much as five steps over lists save against

@@ -253,6 +253,26 @@ def test_autotuned_states_step_over_lists(steps, shrink):
     d.close()
 
 
+def test_first_list_call_while_another_stream_captures():
+    """The allocation of the lists leaves the program's own capture valid."""
+    import torch
+
+    mesh, params, a = _agents(500, 3, 110, 81, 2000)
+    o, d = make_pair(mesh, params, a)
+    _mesh(o)
+    x = torch.zeros(64, device="cuda")
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x += 1
+        d.step(8)
+    o.step(8, 0, 0.0, 0.0)
+    assert_same_state(fetch(d, a), fetch(o, a))
+    graph.replay()
+    graph.replay()
+    assert (x == 2).all().item()
+    d.close()
+
+
 def test_only_calls_over_lists_take_their_memory():
     """200,000 slots: the lists' arrays (some 220 MB) come with the first call
     that steps over lists, not with the state, its uploads or single steps."""
