@@ -521,8 +521,8 @@ int ppc_update_cell_cell_interactions(ppc_state* s, int32_t replicate, ppc_inter
  * next ppc_synchronize or syncing call). Calls of four steps and more run in
  * one launch over neighbour lists that outlive a step, while agents move little
  * enough and the mesh's voxels leave room beside the largest interaction
- * reach; the first such call of a state allocates the lists, about 1.1 KB a
- * slot. All other steps scan the mesh; blocks of them are captured once in a
+ * reach. The lists take about 1.2 KB a slot: of the state's own allocation up
+ * to 100,000 slots, of the first such call's beyond. All other steps scan the mesh; blocks of them are captured once in a
  * CUDA graph and replayed. Both give the same results. */
 
 /* Advances `steps` mechanics steps in the order of simulator::simulate_mechanics

@@ -954,18 +954,20 @@ int replay_steps(ppc_state* s, int k, bool phenotype, double p_divide, double p_
 	return PPC_OK;
 }
 
-// The lists' arrays, about 1.1 KB per slot, made by the first call that uses
-// them: a state that steps once a call, or divides, never does. A device
-// without room for them runs every step through the scanning passes.
-bool lists_allocated(ppc_state* s)
+// The lists' arrays, about 1.2 KB a slot. States of up to kListEarly slots have
+// them in the one block of their arrays (120 MB at most), where they cost next to
+// nothing to allocate; a second block in the first call that uses them takes 0.4
+// to 1 ms, more than a call of 60 steps gains. In larger states, of which many
+// never use them (they divide, settle springs, step once a call), they come with
+// that call. A device without room for them runs every step through the scanning
+// passes.
+constexpr int32_t kListEarly = 100000;
+
+void want_lists(ppc_state* s, arena& a)
 {
-	if (s->lists_tried)
-		return s->lists_fit;
-	s->lists_tried = true;
 	const size_t C = s->total_cap;
 	view& v = s->v;
 	v.nl_pool = 24 * (int64_t)C + 8192;
-	arena a;
 	a.want(v.nl_used, 1);
 	a.want(s->list_bar, 64);
 	a.want(v.lpos[0], C, false);
@@ -979,6 +981,15 @@ bool lists_allocated(ppc_state* s)
 	a.want(v.lspr, C * s->scap, false);
 	a.want(v.lcoef, C * s->scap, false);
 	a.want(v.tpos, C, false);
+}
+
+bool lists_allocated(ppc_state* s)
+{
+	if (s->lists_tried)
+		return s->lists_fit;
+	s->lists_tried = true;
+	arena a;
+	want_lists(s, a);
 	// a capture on another stream of the program stays valid
 	cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
 	cudaThreadExchangeStreamCaptureMode(&mode);
@@ -997,8 +1008,9 @@ constexpr float kSkinUnknown = 1e30f;
 constexpr int kListSteps = 100000; // steps of one launch over lists
 
 // Whether a call's steps run over neighbour lists: the default launch shape or
-// the autotuner's (a caller's choice of another one asks for its own pass), and a mesh that leaves a
-// skin beyond the largest reach (by the uploaded fields). The launch itself
+// the autotuner's (a caller's choice of another one asks for its own pass), and
+// a mesh that leaves a skin beyond the largest reach (by the uploaded fields).
+// The launch itself
 // costs about 13 us over its steps and making lists about as much as one scanning
 // step, so calls of a few steps keep the scanning passes. 88,700 agents, calls of
 // four steps in a row: 48 us a call over lists, 125 scanning; each followed by a
@@ -1337,7 +1349,16 @@ int ppc_create_batch(const ppc_mesh* meshes, const int32_t* capacities, int32_t 
 	a.want(v.moves, 2 * C);
 	a.want(v.nmoves, replicates);
 	a.want(v.draw_epoch, replicates);
-	try_(rc == PPC_OK ? a.place(s) : rc);
+	if (rc == PPC_OK && s->total_cap <= kListEarly)
+	{
+		arena both = a;
+		want_lists(s, both);
+		s->lists_fit = s->lists_tried = both.place(s) == PPC_OK;
+		if (!s->lists_fit)
+			cudaGetLastError(); // the state may fit without them
+	}
+	if (!s->lists_fit)
+		try_(rc == PPC_OK ? a.place(s) : rc);
 	if (rc == PPC_OK)
 	{
 		v.reps = reps;
