@@ -1205,15 +1205,19 @@ __global__ void __launch_bounds__(MOST, 1)
 	lc.pair = reinterpret_cast<double4*>(smem + (T / 32) * sizeof(list_step_warp));
 	lc.entry = reinterpret_cast<int2*>(lc.pair + (size_t)lc.n * T);
 	__shared__ list_barrier bar;
+	__shared__ int s_made, s_debt; // step that the lists in use were made before; their debt
 	if (threadIdx.x == 0)
+	{
 		bar = list_barrier {};
+		s_made = -v.lctl[LCTL_AGE];
+		s_debt = v.lctl[LCTL_DEBT];
+	}
 	__syncthreads();
 	int n = *v.cursor;
 	int p = a.p;
 	float skin = lctl_float(v, LCTL_BUILT);
-	bool past = v.lctl[LCTL_DIRTY] != 0;
+	bool rebuild = v.lctl[LCTL_DIRTY] != 0;
 	const bool cut = lctl_float(v, LCTL_WANT) < skin; // lists that did not fit
-	int age = v.lctl[LCTL_AGE], debt = v.lctl[LCTL_DEBT];
 	if (a.refresh)
 	{
 		unsigned long long ev = 0;
@@ -1222,16 +1226,18 @@ __global__ void __launch_bounds__(MOST, 1)
 		ev = list_wait(v, a, bar, ev);
 		if (ev == ~0ull)
 			return;
-		past = past || ev != 0;
+		rebuild = rebuild || ev != 0;
 	}
-	bool rebuild = past || cut, lists = true;
-	auto charge = [&]() { // lists that lasted `age` steps are to be made anew
-		debt = max(0, debt + kListPays - age);
-		age = 0;
-		lists = debt <= kListDebt;
+	auto charge = [&](int k) { // the lists are to be made anew before step k
+		if (threadIdx.x == 0)
+		{
+			s_debt = max(0, s_debt + kListPays - (k - s_made));
+			s_made = k;
+		}
 	};
-	if (past)
-		charge();
+	if (rebuild)
+		charge(0);
+	rebuild = rebuild || cut;
 	// past this barrier no block reads the control words of the old lists
 	if (rebuild && list_wait(v, a, bar, 0) == ~0ull)
 		return;
@@ -1256,7 +1262,8 @@ __global__ void __launch_bounds__(MOST, 1)
 	{
 		if (rebuild)
 		{
-			if (!list_rebuild<DIMS>(v, a, bar, p, replay, flushed, lists, smem))
+			__syncthreads(); // the debt is thread 0's
+			if (!list_rebuild<DIMS>(v, a, bar, p, replay, flushed, s_debt <= kListDebt, smem))
 				return;
 			n = *v.cursor;
 			skin = lctl_float(v, LCTL_BUILT);
@@ -1286,19 +1293,17 @@ __global__ void __launch_bounds__(MOST, 1)
 				ev |= list_step<DIMS, F32, BATCH>(v, a, reps, lc, w, own, p, t, n, k == 0, last, skin);
 			}
 		p ^= 1;
-		age++;
 		ev = list_wait(v, a, bar, ev);
 		if (ev == ~0ull)
 			return;
 		rebuild = false;
 		if (ev == 0)
 			continue;
-		const bool remove = ev >= kEventRemove;
-		past = (unsigned)(ev >> 32 & 0xffff) != 0;
+		const bool remove = ev >= kEventRemove, past = (unsigned)(ev >> 32 & 0xffff) != 0;
 		replay = remove && a.springs;
 		rebuild = replay || (past && !last);
 		if (rebuild)
-			charge();
+			charge(k + 1);
 		flushed = last;
 		if (past && last && !replay && t0 == 0)
 			v.lctl[LCTL_DIRTY] = 1; // the next call rebuilds first
@@ -1314,8 +1319,8 @@ __global__ void __launch_bounds__(MOST, 1)
 	}
 	if (t0 == 0)
 	{
-		v.lctl[LCTL_AGE] = age;
-		v.lctl[LCTL_DEBT] = debt;
+		v.lctl[LCTL_AGE] = a.steps - s_made;
+		v.lctl[LCTL_DEBT] = s_debt;
 	}
 	if (blockIdx.x == 0 && v.auto_springs)
 		for (int r = threadIdx.x; r < v.nreps; r += T)
