@@ -199,7 +199,8 @@ int ppc_set_random_seed(ppc_state* s, uint64_t seed);
 int ppc_set_launch_shape(ppc_state* s, int32_t tile_edge, int32_t threads, int32_t smem_bytes);
 
 /* How ppc_step runs a mechanics step (ppc_step_with_phenotype and steps with
- * non-zero spring rates always use the separate kernels). */
+ * non-zero spring rates always use kernels of their own; calls over neighbour
+ * lists are one launch in the default form). */
 enum ppc_step_form
 {
 	PPC_STEP_KERNELS = 0,	 /* the default: the fused pass, the compaction plan and

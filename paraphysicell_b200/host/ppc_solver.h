@@ -523,7 +523,7 @@ public:
 	void initialize(environment& e) { containers.initialize(e); }
 
 	// simulator::simulate_mechanics (reference: src/simulator.cpp:157-196)
-	// for `steps` steps in one fused, graph-replayed device call
+	// for `steps` steps in one device call
 	void simulate_mechanics(environment& e, int32_t steps = 1)
 	{
 		once_per_team([&] {
