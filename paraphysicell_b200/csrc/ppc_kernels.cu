@@ -4490,7 +4490,6 @@ static int cooperative_launch(ppc_state* s, void (*k)(view, list_args), int grid
 {
 	a.bar = s->list_bar + 32 * s->bar_set;
 	a.bar_next = s->list_bar + 32 * (s->bar_set ^ 1);
-	s->bar_set ^= 1;
 	cudaLaunchConfig_t cfg {};
 	cfg.gridDim = dim3(grid);
 	cfg.blockDim = dim3(threads);
@@ -4502,6 +4501,7 @@ static int cooperative_launch(ppc_state* s, void (*k)(view, list_args), int grid
 	cfg.attrs = at;
 	cfg.numAttrs = 1;
 	PPC_CUDA(cudaLaunchKernelEx(&cfg, k, s->v, a));
+	s->bar_set ^= 1; // a launch that failed cleared no words
 	return PPC_OK;
 }
 

@@ -426,8 +426,13 @@ extern "C" int ppc_bin_agents_noalloc(const ppc_mesh* mesh, const double* positi
 		if (g_na_stream[dev] != 0 && g_na_stream[dev] != id + 1)
 			PPC_CUDA(cudaStreamWaitEvent(st, g_na_event[dev], 0));
 	}
-	k_na_bins<<<blocks, kNaThreads, 0, st>>>(positions, count, m, voxel_counts, scratch, words, after, agents);
-	PPC_CUDA(cudaGetLastError());
+	// the launch's own status: an error that an earlier call left pending must
+	// not pass for one of this launch, whose words are used up
+	cudaLaunchConfig_t cfg {};
+	cfg.gridDim = dim3(blocks);
+	cfg.blockDim = dim3(kNaThreads);
+	cfg.stream = st;
+	PPC_CUDA(cudaLaunchKernelEx(&cfg, k_na_bins, positions, count, m, voxel_counts, scratch, words, after, agents));
 	if (!captured)
 	{
 		g_na_set[dev] ^= 1;

@@ -142,3 +142,24 @@ def test_all_agents_in_one_voxel():
     torch.cuda.synchronize()
     _check(c)
     assert a.elapsed_time(b) < 35.0
+
+
+def test_an_error_left_by_another_call_is_not_this_ones():
+    """An allocation that failed elsewhere in the program leaves an error
+    pending; a call returns its own status and its own bins, and so does the
+    next one."""
+    import torch
+
+    L = _lib()
+    cases = [_case(5000, 9, 8), _case(90000, 60, 9)]
+    torch.cuda.synchronize()
+    runtime = C.CDLL("libcudart.so.12")
+    for _ in range(3):
+        for c in cases:
+            p = C.c_void_p()
+            assert runtime.cudaMalloc(C.byref(p), C.c_size_t(1 << 60)) != 0
+            try:
+                _call(L, c, torch.cuda.current_stream())
+            finally:
+                runtime.cudaGetLastError()
+            _check(c)
