@@ -967,6 +967,10 @@ void want_lists(ppc_state* s, arena& a)
 {
 	const size_t C = s->total_cap;
 	view& v = s->v;
+	// A warp's lists take as many entries a slot as the longest of them: 16 at one
+	// agent of radius 7 to 10 um per 8,000 um^3 with the full skin, 20 at one per
+	// 6,000, 28 at one per 4,000, whose second attempt, with 0.6 of the skin, takes
+	// 23. Denser tissue gets smaller skins, and beyond one per 3,000 none.
 	v.nl_pool = 24 * (int64_t)C + 8192;
 	a.want(v.nl_used, 1);
 	a.want(s->list_bar, 64);
